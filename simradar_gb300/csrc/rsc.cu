@@ -1056,15 +1056,21 @@ int rsc_set_dff(rsc_worker *w, int slot, const float *icdf, uint32_t n, const fl
     return release_main(w);
 }
 
+/* Most range shells of the spatial order: of 8 type ranges they leave each
+ * a cell per shell. */
+constexpr unsigned kMaxShells = rsc::kMaxSortCells / 32;
+
 static unsigned grid_of(unsigned long long n, unsigned threads) { return (unsigned)((n + threads - 1) / threads); }
 
-/* Counting sort of the background range into spatial order: range shells
- * of a quarter gate, then Morton order of direction, over the scan box
- * (sim_desc s8-s10 origin, s12-s14 size): rsc_sort.cuh.  Every
+/* Counting sort of the type ranges into spatial order, each within itself:
+ * range shells of a quarter gate, LES levels, x, over the scan box (sim_desc
+ * s8-s10 origin, s12-s14 size): rsc_sort.cuh.  Ranges that do not follow one
+ * another leave all but the background in the caller's order.  Every
  * attribute array and perm move to the second buffer set, which then becomes
  * the current one. */
 static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *sim, cudaStream_t st) {
-    const unsigned long long origin = pop->origins[0], count = pop->counts[0];
+    const unsigned long long origin = pop->origins[0];
+    unsigned long long count = pop->counts[0];
     w->sort_due = false;
     w->since_sort = 0;
     if (count < 256 || origin + count > w->num_scats) return RSC_OK;
@@ -1088,10 +1094,7 @@ static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *si
         rsc::k_iota<<<grid_of(numel, rsc::kSortThreads), rsc::kSortThreads, 0, st>>>(w->inv, numel);
         w->launches += 2;
     }
-    /* range shells of a quarter gate over the box's range, direction cells
-     * over its direction cosines, about one scatterer per cell, at most
-     * kMaxSortCells cells */
-    double r_lo = INFINITY, r_hi = 0.0, u_lo = INFINITY, u_hi = -INFINITY, v_lo = INFINITY, v_hi = -INFINITY;
+    double r_lo = INFINITY, r_hi = 0.0;
     for (int c = 0; c < 8; c++) {
         const double x = (double)sim[8] + ((c & 1) ? (double)sim[12] : 0.0);
         const double y = (double)sim[9] + ((c & 2) ? (double)sim[13] : 0.0);
@@ -1100,43 +1103,66 @@ static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *si
         if (!(r > 0.0)) continue;
         r_lo = fmin(r_lo, r);
         r_hi = fmax(r_hi, r);
-        u_lo = fmin(u_lo, x / r);
-        u_hi = fmax(u_hi, x / r);
-        v_lo = fmin(v_lo, z / r);
-        v_hi = fmax(v_hi, z / r);
-    }
-    if (!(r_hi > r_lo) || !(u_hi > u_lo) || !(v_hi > v_lo)) {
-        r_lo = 0.0, r_hi = 1.0, u_lo = -1.0, u_hi = 1.0, v_lo = -1.0, v_hi = 1.0;
     }
     double shell = fabs((double)w->range_delta) * 0.25;
     if (!(shell > 0.0)) shell = (r_hi - r_lo) / 64.0;
     double shells_d = ceil((r_hi - r_lo) / shell);
     if (shells_d < 1.0) shells_d = 1.0;
-    if (shells_d > (double)(rsc::kMaxSortCells / 4)) shells_d = (double)(rsc::kMaxSortCells / 4);
-    const unsigned shells = (unsigned)shells_d;
-    unsigned bits = (unsigned)lrint(0.5 * log2(fmax((double)count / shells, 1.0)));
-    if (bits > 12) bits = 12;
-    while (bits > 0 && ((unsigned long long)shells << (2 * bits)) > rsc::kMaxSortCells) bits--;
-    const unsigned H = shells << (2 * bits);
+    if (shells_d > (double)kMaxShells) shells_d = (double)kMaxShells;
+    a.shells = (unsigned)shells_d;
+    /* the LES levels the box meets */
+    float lo3[3], hi3[3];
+    rsc::wind_table_index(lo3, make_float4(0.0f, 0.0f, sim[10], 0.0f), w->les_desc, sim);
+    rsc::wind_table_index(hi3, make_float4(0.0f, 0.0f, sim[10] + sim[14], 0.0f), w->les_desc, sim);
+    double k_lo = floor((double)lo3[2] - 0.5), k_n = floor((double)hi3[2] - 0.5) - k_lo + 1.0;
+    if (!(k_n >= 1.0 && k_n <= 65536.0)) k_lo = 0.0, k_n = 1.0;
+    /* rows (a level of a shell) of about 128 scatterers or more, cells of
+     * about one, the types sharing kMaxSortCells in proportion */
+    unsigned H = 0;
+    unsigned long long before = 0;
+    for (int t = 0; t < a.nranges; t++) {
+        rsc::SortRange &R = a.range[t];
+        const double n = (double)(R.end - before), per_shell = n / a.shells;
+        const double most = fmax(1.0, floor((double)(rsc::kMaxSortCells - a.nranges * a.shells) * (n / count) / a.shells));
+        const double levels = fmax(1.0, fmin(fmin(k_n, floor(per_shell / 128.0)), most));
+        const double cells = fmax(1.0, fmin(per_shell / levels, floor(most / levels)));
+        R.levels = (unsigned)levels;
+        R.cells = (unsigned)cells;
+        R.base = H;
+        H += a.shells * R.levels * R.cells;
+        before = R.end;
+    }
     RSC_CUDA(cudaMemsetAsync(w->sort_hist, 0, H * sizeof(unsigned), st));
-    rsc::SortArgs a;
     a.pos = w->pos;
     a.origin = origin;
     a.count = count;
     a.r0 = (float)r_lo;
-    a.ir = (float)(1.0 / (shells * shell));
-    a.u0 = (float)u_lo;
-    a.iu = (float)(1.0 / (u_hi - u_lo));
-    a.v0 = (float)v_lo;
-    a.iv = (float)(1.0 / (v_hi - v_lo));
-    a.shells = shells;
-    a.bits = bits;
+    a.ir = (float)(1.0 / (shells_d * shell));
+    a.x0 = sim[8];
+    a.ix = sim[12] > 0.0f ? 1.0f / sim[12] : 0.0f;
+    a.k0 = (float)k_lo;
+    a.ik = (float)(1.0 / k_n);
+    memcpy(a.wind, w->les_desc, sizeof(a.wind));
+    memcpy(a.sim, sim, sizeof(a.sim));
     a.key = w->sort_key;
     a.hist = w->sort_hist;
     rsc::k_sort_key<<<grid_of(count, rsc::kSortThreads), rsc::kSortThreads, 0, st>>>(a);
     const unsigned nb = (H + rsc::kScanBlock - 1) / rsc::kScanBlock;
     rsc::k_scan_blocks<<<nb, rsc::kScanThreads, 0, st>>>(w->sort_hist, H, w->sort_blocks);
     rsc::k_scan_top<<<1, rsc::kScanThreads, 0, st>>>(w->sort_blocks, nb);
+    rsc::SortArgs a;
+    a.nranges = 1;
+    a.range[0].end = count;
+    for (int k = 1; k < RSC_MAX_TYPES; k++) {
+        if (pop->counts[k] == 0) continue;
+        if (pop->origins[k] != origin + count) {
+            count = pop->counts[0];
+            a.nranges = 1;
+            break;
+        }
+        count += pop->counts[k];
+        a.range[a.nranges++].end = count;
+    }
     rsc::k_scan_add<<<nb, rsc::kScanThreads, 0, st>>>(w->sort_hist, H, w->sort_blocks);
     rsc::k_sort_scatter<<<grid_of(count, rsc::kSortThreads), rsc::kSortThreads, 0, st>>>(w->sort_key, count,
                                                                                         w->sort_hist, w->sort_order);
@@ -1178,6 +1204,7 @@ static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *si
 static int settle_sig_aux(rsc_worker *w, cudaStream_t st) {
     if (!w->sig_aux_stale || !w->have_pulse_desc) return RSC_OK;
     PulseArgs P;
+    if (!(r_hi > r_lo)) r_lo = 0.0, r_hi = 1.0;
     fill_pulse_args(w, P, w->last_sim);
     if (w->sa_pos != nullptr) {
         P.pos = w->sa_pos;

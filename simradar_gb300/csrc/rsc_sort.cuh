@@ -1,10 +1,10 @@
 /*
- * rsc_sort.cuh -- spatial order of the background scatterers.
+ * rsc_sort.cuh -- spatial order of the scatterers.
  *
  * Scatterers are independent: where one sits in the attribute arrays changes
- * nothing in its evolution.  The worker may therefore keep the background
- * range in spatial order (range shells, then Morton order of direction),
- * which makes a warp's 32 scatterers neighbours in space: their range-gate candidates
+ * nothing in its evolution.  The worker may therefore keep every type's
+ * range in spatial order (range shells, then LES levels, then x), which makes
+ * a warp's 32 scatterers neighbours in space: their range-gate candidates
  * coincide (the pulse kernel then sums each gate across the warp instead of
  * with per-lane atomics) and their LES texels overlap (the advance kernel's
  * gathers hit L1).  The order is restored by a counting sort every few
@@ -26,6 +26,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "rsc_physics.cuh"
+
 namespace rsc {
 
 constexpr unsigned kSortThreads = 256;
@@ -34,16 +36,6 @@ constexpr unsigned kScanPerThread = 4;
 constexpr unsigned kScanBlock = kScanThreads * kScanPerThread;   /* histogram entries per scan block */
 constexpr unsigned kMaxSortCells = 1u << 22;                     /* histogram entries */
 
-/* the 16 low bits of v spread to every second bit (2-D Morton order) */
-__device__ __forceinline__ unsigned morton_spread(unsigned v) {
-    v &= 0xffffu;
-    v = (v | (v << 8)) & 0x00ff00ffu;
-    v = (v | (v << 4)) & 0x0f0f0f0fu;
-    v = (v | (v << 2)) & 0x33333333u;
-    v = (v | (v << 1)) & 0x55555555u;
-    return v;
-}
-
 /* cell of x among `cells` equal cells covering [o, o + 1 / inv_len) */
 __device__ __forceinline__ unsigned cell_axis(float x, float o, float inv_size, float cells) {
     float f = (x - o) * inv_size * cells;
@@ -51,17 +43,24 @@ __device__ __forceinline__ unsigned cell_axis(float x, float o, float inv_size, 
     return (unsigned)f;
 }
 
-/* Cells are range-major: shells of a quarter gate in range, each divided
- * in 2^bits x 2^bits direction cells (the direction cosines x / r and z / r
- * over the box) in Morton order.  A warp's scatterers then share a range
- * shell (so they reach the same few gates) and a small patch of directions
- * (so their LES texels are neighbours). */
+/* Cells are ordered by type range (each stays where it is), range shell,
+ * level of the LES grid (the vertical texel cell, or groups of them), and x.
+ * A warp's scatterers then lie in one shell (they reach the same few gates)
+ * and in a short run of x inside a level (their LES texels share lines). */
+struct SortRange {
+    unsigned long long end;            /* of the type's range, from the first range's start */
+    unsigned base, levels, cells;      /* first cell, LES levels, cells of x */
+};
 struct SortArgs {
     const float4 *pos;
     unsigned long long origin, count;
     float r0, ir;          /* range covered by the shells: start, 1 / length */
-    float u0, iu, v0, iv;  /* x / r and z / r covered by the cells: start, 1 / length */
-    unsigned shells, bits;
+    float x0, ix;          /* x covered by the cells of a row: start, 1 / length */
+    float k0, ik;          /* LES levels covered: start, 1 / number */
+    unsigned shells;
+    int nranges;
+    SortRange range[8];
+    float wind[16], sim[16];
     unsigned *key;
     unsigned *hist;
 };
@@ -69,14 +68,17 @@ struct SortArgs {
 __global__ void __launch_bounds__(kSortThreads) k_sort_key(const SortArgs a) {
     const unsigned long long i = (unsigned long long)blockIdx.x * kSortThreads + threadIdx.x;
     if (i >= a.count) return;
+    int t = 0;
+    while (t + 1 < a.nranges && i >= a.range[t].end) t++;
+    const SortRange &R = a.range[t];
     const float4 p = a.pos[a.origin + i];
     const float r = sqrtf(p.x * p.x + p.y * p.y + p.z * p.z);
-    const float ri = r > 0.0f ? 1.0f / r : 0.0f;
+    float c[3];
+    wind_table_index(c, p, a.wind, a.sim);
     const unsigned sh = cell_axis(r, a.r0, a.ir, (float)a.shells);
-    const float cells = (float)(1u << a.bits);
-    const unsigned cu = cell_axis(p.x * ri, a.u0, a.iu, cells);
-    const unsigned cv = cell_axis(p.z * ri, a.v0, a.iv, cells);
-    const unsigned code = (sh << (2 * a.bits)) | morton_spread(cu) | (morton_spread(cv) << 1);
+    const unsigned lv = cell_axis(floorf(c[2] - 0.5f), a.k0, a.ik, (float)R.levels);
+    const unsigned cx = cell_axis(p.x, a.x0, a.ix, (float)R.cells);
+    const unsigned code = R.base + (sh * R.levels + lv) * R.cells + cx;
     a.key[i] = code;
     atomicAdd(a.hist + code, 1u);
 }
