@@ -493,7 +493,8 @@ int rsc_make_pulse_noalloc(const float *pos4, const float *rcs4, size_t num_scat
  * on the triangle table {0, 1, 0} with scale b, origin 1, max 2; 9 / 10
  * the error (against double) of the compensated pulse's double-float sine /
  * cosine of the two-way phase b a for a range a and a wave number b,
- * 11 / 12 the same for the plain FP32 form.  Host arrays of n floats. */
+ * 11 / 12 the same for the plain FP32 form; 13 the mid-range square root, 14
+ * the mid-range quotient a / b.  Host arrays of n floats. */
 int rsc_eval_math(int fn, const float *a, const float *b, float *out, size_t n);
 
 #ifdef __cplusplus

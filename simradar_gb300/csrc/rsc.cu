@@ -86,6 +86,7 @@ struct rsc_worker {
     double *pulse64 = nullptr;
     float *rk = nullptr, *rk_hi = nullptr, *rk_lo = nullptr;
     double *rk64 = nullptr;
+    float *node = nullptr;        /* node positions -kNodeMaxN .. G - 1 + kNodeMaxN (rsc_nodes.cuh) */
     double *acc64 = nullptr;      /* the pulse kernel's FP64 grid accumulator */
     unsigned *counter = nullptr;
     unsigned long long *runs = nullptr;   /* the compensated pulse's run counter */
@@ -138,6 +139,7 @@ struct rsc_worker {
      * caller's index, inv[index] the slot; NULL perm = caller's order */
     int sort_interval = 128;
     uint64_t since_sort = 0;
+    uint64_t sort_end = 0;    /* slots [0, sort_end) are in spatial order */
     bool sort_due = true;
     unsigned *perm = nullptr, *perm_alt = nullptr, *inv = nullptr;
     unsigned *sort_key = nullptr, *sort_order = nullptr, *sort_hist = nullptr, *sort_blocks = nullptr;
@@ -162,7 +164,7 @@ struct rsc_worker {
     bool read_pending = false, read_next_pending = false, main_pending = false;
     uint64_t adv_seq = 0, adv_joined = 0;   /* work queued on adv / covered by the last join */
     /* the last pulse launch shape: mode, path, gates, tuning -> grid, threads, smem */
-    int geo_key[5] = {-1, -1, -1, -1, -1};
+    int geo_key[6] = {-1, -1, -1, -1, -1, -1};
     int geo_grid = 0, geo_threads = 0;
     size_t geo_smem = 0;
     /* rsc_download_pulse_async: the pulse goes to the host on its own stream,
@@ -279,6 +281,7 @@ void free_arrays(rsc_worker *w) {
     free_ptr(w->rk_hi);
     free_ptr(w->rk_lo);
     free_ptr(w->rk64);
+    free_ptr(w->node);
     free_ptr(w->acc64);
     free_ptr(w->counter);
     free_ptr(w->runs);
@@ -288,6 +291,7 @@ void free_arrays(rsc_worker *w) {
     w->pulse64 = nullptr;
     w->rk = w->rk_hi = w->rk_lo = nullptr;
     w->rk64 = nullptr;
+    w->node = nullptr;
     w->acc64 = nullptr;
     w->counter = nullptr;
     w->runs = nullptr;
@@ -394,6 +398,9 @@ int fill_debris(rsc_worker *w, const rsc_population *pop, AdvanceArgs &a, unsign
     return RSC_OK;
 }
 
+/* float4 of the nodes' single-scatterer sums: node_copies() copies */
+constexpr size_t kStrayFloat4s = 1024;
+
 /* Gate origins: the FP32 running sum of make_pulse_pass_1 (rs.cl:1214) and
  * the FP64 values range_start + k * range_delta (head and tail). */
 int set_gates(rsc_worker *w) {
@@ -413,6 +420,13 @@ int set_gates(rsc_worker *w) {
     RSC_CUDA(cudaMemcpy(w->rk_hi, hi.data(), G * sizeof(float), cudaMemcpyHostToDevice));
     RSC_CUDA(cudaMemcpy(w->rk_lo, lo.data(), G * sizeof(float), cudaMemcpyHostToDevice));
     RSC_CUDA(cudaMemcpy(w->rk64, r64.data(), G * sizeof(double), cudaMemcpyHostToDevice));
+    /* the nodes: the running sum's origins, continued evenly on both sides */
+    std::vector<float> nd(rsc::node_count(G, rsc::kNodeMaxN));
+    for (int m = -rsc::kNodeMaxN; m < (int)G + rsc::kNodeMaxN; m++) {
+        const int k = std::min(std::max(m, 0), (int)G - 1);
+        nd[m + rsc::kNodeMaxN] = (float)((double)rk[k] + (double)(m - k) * (double)w->range_delta);
+    }
+    RSC_CUDA(cudaMemcpy(w->node, nd.data(), nd.size() * sizeof(float), cudaMemcpyHostToDevice));
     return RSC_OK;
 }
 
@@ -446,6 +460,7 @@ typedef void (*PulseKernel)(const PulseArgs);
  * the path at run time (one compensated kernel per path measured 7% slower). */
 PulseKernel pulse_kernel(int mode, int path) {
     if (mode == RSC_PULSE_PLAIN) {
+        if (path == 5) return rsc::k_pulse_nodes;
         if (path == 4) return rsc::k_pulse_group<0, kPulseGroup, 1>;
         if (path == 3) return rsc::k_pulse_group<0, kPulseGroup>;
         return path == 2 ? rsc::k_pulse<0, 2> : (path == 1 ? rsc::k_pulse<0, 1> : rsc::k_pulse<0, 0>);
@@ -462,18 +477,38 @@ PulseKernel pulse_kernel(int mode, int path) {
  * when it does not write aux / sig), 4 the same with the triangle range
  * table compiled in */
 int pulse_path(const PulseArgs &P, int mode) {
+    if (mode == RSC_PULSE_PLAIN && P.mom_n > 0) return 5;
     if (P.dense) return 2;
     if (P.coherent_span <= 0) return 0;
     if ((mode == RSC_PULSE_PLAIN && !P.materialize) || mode == RSC_PULSE_COMPENSATED) return P.rw_tri ? 4 : 3;
     return 1;
 }
 
+/* Resident blocks per SM of the node form's pulse: one fewer than fit leave
+ * the advance of the same step its share of the SM (README scale, a dwell of
+ * 10 pulses: 580 us with 3, 592 with 4, 588 with 2). */
+constexpr int kNodePerSm = 3;
+
 /* Launch shape of the pulse kernel (one-instance or batched form) for G
  * gates: warps per block as many as fit 200 KB of bins (at most 16, at most
  * want_warps when that is > 0), resident blocks per SM from the occupancy
  * calculator (at most 4, at most want_per_sm when that is > 0). */
 int pulse_shape(int mode, bool batch, uint32_t G, int want_warps, int want_per_sm, int *per_sm_out, int *threads,
-                size_t *smem, int path = 0) {
+                size_t *smem, int path = 0, int mom_n = 0) {
+    if (path == 5) {
+        const int warps = rsc::kNodeThreads / 32;
+        *threads = 32 * (want_warps > 0 && want_warps < warps ? want_warps : warps);
+        *smem = rsc::node_smem_bytes(G, mom_n);
+        int fit = 1;
+        cudaError_t e = batch ? kernel_occupancy(rsc::k_pulse_batch_nodes, *threads, *smem, &fit)
+                              : kernel_occupancy(pulse_kernel(mode, path), *threads, *smem, &fit);
+        if (e != cudaSuccess) return cuda_fail(RSC_ERR_CUDA, "pulse kernel configuration: %s", cudaGetErrorString(e));
+        if (want_per_sm <= 0) want_per_sm = kNodePerSm;
+        if (fit < 1) fit = 1;
+        if (want_per_sm < fit) fit = want_per_sm;
+        *per_sm_out = fit;
+        return RSC_OK;
+    }
     size_t per_warp = rsc::pulse_warp_bytes(mode, G);
     size_t budget = 200 * 1024;
     int warps = (int)(budget / per_warp);
@@ -510,8 +545,14 @@ int pulse_shape(int mode, bool batch, uint32_t G, int want_warps, int want_per_s
     return RSC_OK;
 }
 
-int pulse_geometry(rsc_worker *w, int mode, int path, int *grid, int *threads, size_t *smem) {
-    const int key[5] = {mode, path, (int)w->G, w->tune_warps, w->tune_per_sm};
+/* Blocks that a state of n scatterers keeps busy in the node form. */
+int node_grid(unsigned long long n, int threads) {
+    const unsigned long long per_block = 64ull * rsc::kNodeRuns * (unsigned)(threads / 32);
+    return (int)std::min<unsigned long long>(std::max<unsigned long long>((n + per_block - 1) / per_block, 1), 1u << 20);
+}
+
+int pulse_geometry(rsc_worker *w, int mode, int path, int mom_n, int *grid, int *threads, size_t *smem) {
+    const int key[6] = {mode, path, (int)w->G, w->tune_warps, w->tune_per_sm, mom_n};
     if (memcmp(key, w->geo_key, sizeof(key)) == 0) {
         /* same shape as the last launch: no occupancy query per pulse */
         *grid = w->geo_grid;
@@ -520,7 +561,7 @@ int pulse_geometry(rsc_worker *w, int mode, int path, int *grid, int *threads, s
         return RSC_OK;
     }
     int per_sm = 1;
-    int s = pulse_shape(mode, false, w->G, w->tune_warps, w->tune_per_sm, &per_sm, threads, smem, path);
+    int s = pulse_shape(mode, false, w->G, w->tune_warps, w->tune_per_sm, &per_sm, threads, smem, path, mom_n);
     if (s) return s;
     *grid = w->num_sms * per_sm;
     memcpy(w->geo_key, key, sizeof(key));
@@ -595,6 +636,16 @@ int moment_span(const PulseArgs &P) {
     return (int)n;
 }
 
+/* Half width of the triangle range weight in gate spacings when that is a
+ * whole number the node sums take (rsc_nodes.cuh), else 0. */
+int node_span(const PulseArgs &P) {
+    if (!P.rw_tri || !(P.rdelta > 0.0f) || !(P.rwd[0] > 0.0f)) return 0;
+    const double x = 1.0 / ((double)P.rwd[0] * (double)P.rdelta);
+    const double n = floor(x + 0.5);
+    if (n < 1.0 || n > (double)rsc::kNodeMaxN || fabs(x - n) > 1.0e-6 * n) return 0;
+    return (int)n;
+}
+
 /* The margin, in gates, by which the sparse path widens the exact support
  * d_lo .. d_hi (metres) of the range weight: the measured drift of the FP32
  * running-sum gate origins from exact spacing; two ulps of the largest range
@@ -608,6 +659,17 @@ double window_margin(double drift, float range_start, float range_delta, uint32_
     const double r_max = fabs((double)range_start) + delta * span;
     const double ulp_r = ldexp(1.0, ilogb(r_max) - 23);
     return (drift + 2.0 * ulp_r) / delta + 8.0 * ldexp(1.0, -23) * span + 1.0e-4;
+}
+
+/* The plain pulse through the node sums where the triangle allows them: a
+ * state in spatial order, or a triangle too wide for the gate window. */
+void use_nodes(rsc_worker *w, PulseArgs &P) {
+    const int n = node_span(P);
+    if (n == 0 || (P.coherent_span <= 0 && !P.dense)) return;
+    P.mom_n = n;
+    P.node = w->node + (rsc::kNodeMaxN - n);
+    P.stray = reinterpret_cast<float4 *>(w->acc64 + (rsc::node_count(w->G, rsc::kNodeMaxN) + w->G) * 4);
+    P.lead = w->perm != nullptr ? w->sort_end : 0;
 }
 
 void fill_pulse_args(rsc_worker *w, PulseArgs &P, const float *sim) {
@@ -811,9 +873,13 @@ int rsc_worker_malloc(rsc_worker *w, size_t num_scats, float range_start, float 
     RSC_CUDA(cudaMalloc((void **)&w->rk_hi, range_count * sizeof(float)));
     RSC_CUDA(cudaMalloc((void **)&w->rk_lo, range_count * sizeof(float)));
     RSC_CUDA(cudaMalloc((void **)&w->rk64, range_count * sizeof(double)));
-    /* the pulse kernel's FP64 accumulator; each launch leaves it at zero */
-    RSC_CUDA(cudaMalloc((void **)&w->acc64, range_count * 4 * sizeof(double)));
-    RSC_CUDA(cudaMemsetAsync(w->acc64, 0, range_count * 4 * sizeof(double), w->stream));
+    const size_t nodes = rsc::node_count(range_count, rsc::kNodeMaxN);
+    RSC_CUDA(cudaMalloc((void **)&w->node, nodes * sizeof(float)));
+    /* the pulse kernels' FP64 accumulator (gates, or nodes and then gates);
+     * each launch leaves it at zero */
+    const size_t acc_bytes = (nodes + range_count) * 4 * sizeof(double) + kStrayFloat4s * sizeof(float4);
+    RSC_CUDA(cudaMalloc((void **)&w->acc64, acc_bytes));
+    RSC_CUDA(cudaMemsetAsync(w->acc64, 0, acc_bytes, w->stream));
     RSC_CUDA(cudaMalloc((void **)&w->counter, sizeof(unsigned)));
     RSC_CUDA(cudaMemsetAsync(w->counter, 0, sizeof(unsigned), w->stream));
     RSC_CUDA(cudaMalloc((void **)&w->runs, sizeof(unsigned long long)));
@@ -1073,6 +1139,19 @@ static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *si
     unsigned long long count = pop->counts[0];
     w->sort_due = false;
     w->since_sort = 0;
+    rsc::SortArgs a;
+    a.nranges = 1;
+    a.range[0].end = count;
+    for (int k = 1; k < RSC_MAX_TYPES; k++) {
+        if (pop->counts[k] == 0) continue;
+        if (pop->origins[k] != origin + count) {
+            count = pop->counts[0];
+            a.nranges = 1;
+            break;
+        }
+        count += pop->counts[k];
+        a.range[a.nranges++].end = count;
+    }
     if (count < 256 || origin + count > w->num_scats) return RSC_OK;
     const unsigned long long numel = w->numel;
     if (w->perm == nullptr) {
@@ -1104,6 +1183,7 @@ static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *si
         r_lo = fmin(r_lo, r);
         r_hi = fmax(r_hi, r);
     }
+    if (!(r_hi > r_lo)) r_lo = 0.0, r_hi = 1.0;
     double shell = fabs((double)w->range_delta) * 0.25;
     if (!(shell > 0.0)) shell = (r_hi - r_lo) / 64.0;
     double shells_d = ceil((r_hi - r_lo) / shell);
@@ -1150,19 +1230,6 @@ static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *si
     const unsigned nb = (H + rsc::kScanBlock - 1) / rsc::kScanBlock;
     rsc::k_scan_blocks<<<nb, rsc::kScanThreads, 0, st>>>(w->sort_hist, H, w->sort_blocks);
     rsc::k_scan_top<<<1, rsc::kScanThreads, 0, st>>>(w->sort_blocks, nb);
-    rsc::SortArgs a;
-    a.nranges = 1;
-    a.range[0].end = count;
-    for (int k = 1; k < RSC_MAX_TYPES; k++) {
-        if (pop->counts[k] == 0) continue;
-        if (pop->origins[k] != origin + count) {
-            count = pop->counts[0];
-            a.nranges = 1;
-            break;
-        }
-        count += pop->counts[k];
-        a.range[a.nranges++].end = count;
-    }
     rsc::k_scan_add<<<nb, rsc::kScanThreads, 0, st>>>(w->sort_hist, H, w->sort_blocks);
     rsc::k_sort_scatter<<<grid_of(count, rsc::kSortThreads), rsc::kSortThreads, 0, st>>>(w->sort_key, count,
                                                                                         w->sort_hist, w->sort_order);
@@ -1190,6 +1257,12 @@ static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *si
     w->perm_alt = t;
     rsc::k_sort_inverse<<<grid_of(numel, rsc::kSortThreads), rsc::kSortThreads, 0, st>>>(w->perm, w->inv, numel);
     RSC_CUDA(cudaGetLastError());
+    /* ranges dense enough for a run of 64 to lie in a few shells */
+    w->sort_end = 0;
+    for (int t = 0; t < a.nranges && origin == 0; t++) {
+        if (a.range[t].end - w->sort_end < 8ull * a.shells) break;
+        w->sort_end = a.range[t].end;
+    }
     w->launches += 8;
     w->sorts++;
     return RSC_OK;
@@ -1204,7 +1277,6 @@ static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *si
 static int settle_sig_aux(rsc_worker *w, cudaStream_t st) {
     if (!w->sig_aux_stale || !w->have_pulse_desc) return RSC_OK;
     PulseArgs P;
-    if (!(r_hi > r_lo)) r_lo = 0.0, r_hi = 1.0;
     fill_pulse_args(w, P, w->last_sim);
     if (w->sa_pos != nullptr) {
         P.pos = w->sa_pos;
@@ -1616,10 +1688,12 @@ int rsc_make_pulse(rsc_worker *w, const float sim_desc[16]) {
     }
     const bool mat = (mode == RSC_PULSE_PLAIN) && (w->materialize || sim_desc[15] != 0.0f);
     P.materialize = mat ? 1 : 0;
+    if (mode == RSC_PULSE_PLAIN && !mat && !w->pend) use_nodes(w, P);
     int grid = 0, threads = 0;
     size_t smem = 0;
-    s = pulse_geometry(w, mode, pulse_path(P, mode), &grid, &threads, &smem);
+    s = pulse_geometry(w, mode, pulse_path(P, mode), P.mom_n, &grid, &threads, &smem);
     if (s) return s;
+    if (pulse_path(P, mode) == 5) grid = std::min(grid, node_grid(P.n, threads));
     s = pulse_d2h_wait(w);
     if (s) return s;
     if (w->pend && mode != RSC_PULSE_F64) {
@@ -1794,6 +1868,7 @@ struct rsc_batch {
      * (0: as many as fit) */
     int adv_threads = rsc::kAdvanceThreads, adv_per_sm = 0;
     size_t adv_smem = 0;
+    bool nodes = false; /* the plain pulse through the node sums */
     bool tri = false;   /* the pulse kernel with the triangle range weight compiled in */
     /* per-instance launch descriptors and block prefixes */
     std::vector<rsc::BatchAdvance> h_adv;
@@ -1880,11 +1955,8 @@ int batch_reserve(rsc_batch *b, int steps) {
 int batch_prepare(rsc_batch *b, const rsc::BatchStep *row) {
     if (!b->have_pops) return fail(RSC_ERR_STATE, "rsc_batch_set_populations has not been called");
     const size_t n = b->w.size();
-    int per_sm = 1, threads = 0;
+    int per_sm = 1, threads = 0, s = RSC_OK;
     size_t smem = 0;
-    int s = pulse_shape(b->mode, true, b->Gmax, b->tune_warps, b->tune_per_sm, &per_sm, &threads, &smem);
-    if (s) return s;
-    const double total = (double)b->num_sms * per_sm;
     double sum_n = 0.0;
     for (rsc_worker *x : b->w) sum_n += (double)x->num_scats;
     b->h_adv.assign(n, rsc::BatchAdvance());
@@ -1895,6 +1967,8 @@ int batch_prepare(rsc_batch *b, const rsc::BatchStep *row) {
     bool tri = true;   /* every instance's range table is the triangle */
     b->concept.assign(n, 0u);
     unsigned acc_r = 0, acc_d = 0, acc_p = 0;
+    bool nodes = true;
+    int max_n = 0;
     for (size_t i = 0; i < n; i++) {
         rsc_worker *x = b->w[i];
         if (x->pos == nullptr) return fail(RSC_ERR_STATE, "instance %zu is not allocated", i);
@@ -1928,26 +2002,39 @@ int batch_prepare(rsc_batch *b, const rsc::BatchStep *row) {
             P.runs = x->runs;
         }
         P.materialize = 0;
+        if (b->mode == RSC_PULSE_PLAIN) use_nodes(x, P);
+        nodes = nodes && P.mom_n > 0;
+        max_n = std::max(max_n, P.mom_n);
         tri = tri && P.rw_tri;
+        b->concept[i] = rsm_f2u(row[i].sim[5]);
+    }
+    /* the plain pulse through the node sums when every instance's may */
+    nodes = nodes && b->mode == RSC_PULSE_PLAIN;
+    s = pulse_shape(b->mode, true, b->Gmax, b->tune_warps, b->tune_per_sm, &per_sm, &threads, &smem, nodes ? 5 : 0, max_n);
+    if (s) return s;
+    const double total = (double)b->num_sms * per_sm;
+    for (size_t i = 0; i < n; i++) {
+        rsc_worker *x = b->w[i];
         /* pulse blocks in proportion to the scatterers, at least one, and no
          * block without a scatterer to start on */
         double share = sum_n > 0.0 ? total * (double)x->num_scats / sum_n : 1.0;
         unsigned bi = (unsigned)llround(share);
         unsigned cap = (unsigned)((x->num_scats + (size_t)threads - 1) / (size_t)threads);
+        if (nodes) cap = (unsigned)node_grid(x->num_scats, threads);
         if (bi > cap) bi = cap;
         if (bi < 1) bi = 1;
         b->h_pulse_prefix[i] = acc_p;
         acc_p += bi;
-        b->concept[i] = rsm_f2u(row[i].sim[5]);
     }
     b->h_rain_prefix[n] = acc_r;
     b->h_deb_prefix[n] = acc_d;
     b->h_pulse_prefix[n] = acc_p;
     if (acc_r != b->rain_blocks || acc_d != b->deb_blocks || acc_p != b->pulse_blocks || threads != b->pulse_threads ||
-        smem != b->pulse_smem || tri != b->tri) {
+        smem != b->pulse_smem || tri != b->tri || nodes != b->nodes) {
         batch_drop_graph(b);
     }
     b->tri = tri;
+    b->nodes = nodes;
     b->rain_blocks = acc_r;
     b->deb_blocks = acc_d;
     b->pulse_blocks = acc_p;
@@ -1972,7 +2059,9 @@ cudaError_t batch_launch_pulse(rsc_batch *b, int k) {
     float4 *out = b->d_out + (size_t)k * n * b->Gmax;
     const unsigned g = b->pulse_blocks, t = (unsigned)b->pulse_threads;
     const size_t sm = b->pulse_smem;
-    if (b->mode == RSC_PULSE_PLAIN && b->tri) {
+    if (b->nodes) {
+        rsc::k_pulse_batch_nodes<<<g, t, sm, b->stream>>>(b->d_pulse, st, b->d_pulse_prefix, n, out, b->Gmax);
+    } else if (b->mode == RSC_PULSE_PLAIN && b->tri) {
         rsc::k_pulse_batch<0, 1><<<g, t, sm, b->stream>>>(b->d_pulse, st, b->d_pulse_prefix, n, out, b->Gmax);
     } else if (b->mode == RSC_PULSE_PLAIN) {
         rsc::k_pulse_batch<0><<<g, t, sm, b->stream>>>(b->d_pulse, st, b->d_pulse_prefix, n, out, b->Gmax);
@@ -2210,6 +2299,7 @@ int rsc_autotune(rsc_worker *w, const float sim_desc[16], int *warps_out, int *b
         P.runs = w->runs;
     }
     P.materialize = 0;
+    if (mode == RSC_PULSE_PLAIN) use_nodes(w, P);
     s = pulse_d2h_wait(w);
     if (s) return s;
     EventPair ev;
@@ -2220,7 +2310,8 @@ int rsc_autotune(rsc_worker *w, const float sim_desc[16], int *warps_out, int *b
         for (int per_sm = 1; per_sm <= 4; per_sm++) {
             int got = 0, threads = 0;
             size_t smem = 0;
-            s = pulse_shape(mode, false, w->G, warps, per_sm, &got, &threads, &smem, pulse_path(P, mode));
+            s = pulse_shape(mode, false, w->G, warps, per_sm, &got, &threads, &smem, pulse_path(P, mode),
+                            P.mom_n);
             if (s) return s;
             if (threads != warps * 32 || got != per_sm) continue;   /* shape not reachable */
             const int grid = w->num_sms * per_sm;

@@ -19,6 +19,7 @@
 #define SIMRADAR_GB300_RSC_BATCH_CUH
 
 #include "rsc_step.cuh"
+#include "rsc_nodes.cuh"
 
 namespace rsc {
 
@@ -131,13 +132,10 @@ k_advance_batch_debris(const BatchAdvance *inst, const BatchStep *steps, const u
     debris_step(sa, T, (size_t)(T.origin + (j - sa.deb_prefix[t])), pos, rcs, known);
 }
 
-/* TRI 1: every instance's range table is the triangle (compiled in) */
-template <int MODE, int TRI = -1>
-__global__ void __launch_bounds__(512)
-k_pulse_batch(const PulseArgs *inst, const BatchStep *steps, const unsigned *prefix, int ninst, float4 *out,
-              unsigned out_stride) {
-    __shared__ __align__(16) PulseArgs sp;
-    __shared__ int s_i;
+/* The instance of this block and its pulse descriptor for the step, in
+ * shared memory; returns the instance. */
+__device__ __forceinline__ int batch_pulse_args(PulseArgs &sp, int &s_i, const PulseArgs *inst, const BatchStep *steps,
+                                                const unsigned *prefix, int ninst, float4 *out, unsigned out_stride) {
     if (threadIdx.x == 0) s_i = batch_instance(prefix, ninst, blockIdx.x);
     __syncthreads();
     const int i = s_i;
@@ -151,6 +149,28 @@ k_pulse_batch(const PulseArgs *inst, const BatchStep *steps, const unsigned *pre
         beam_norm_df(steps[i].sim, sp.bn_hi, sp.bn_lo);
     }
     __syncthreads();
+    return i;
+}
+
+/* Every instance's plain pulse through its node sums (rsc_nodes.cuh). */
+__global__ void __launch_bounds__(kNodeThreads, kNodeMinBlocks)
+k_pulse_batch_nodes(const PulseArgs *inst, const BatchStep *steps, const unsigned *prefix, int ninst, float4 *out,
+                    unsigned out_stride) {
+    __shared__ __align__(16) PulseArgs sp;
+    __shared__ int s_i;
+    const int i = batch_pulse_args(sp, s_i, inst, steps, prefix, ninst, out, out_stride);
+    const unsigned b0 = __ldg(prefix + i);
+    node_body(sp, blockIdx.x - b0, __ldg(prefix + i + 1) - b0);
+}
+
+/* TRI 1: every instance's range table is the triangle (compiled in) */
+template <int MODE, int TRI = -1>
+__global__ void __launch_bounds__(512)
+k_pulse_batch(const PulseArgs *inst, const BatchStep *steps, const unsigned *prefix, int ninst, float4 *out,
+              unsigned out_stride) {
+    __shared__ __align__(16) PulseArgs sp;
+    __shared__ int s_i;
+    const int i = batch_pulse_args(sp, s_i, inst, steps, prefix, ninst, out, out_stride);
     const unsigned b0 = __ldg(prefix + i);
     /* an instance whose state is in spatial order takes two scatterers per
      * lane, as the one-instance kernel does */

@@ -479,6 +479,9 @@ struct PulseArgs {
                           * summed per range interval as moments (PulseBins::add_k), 0 otherwise */
     double *acc64;       /* G * 4 FP64 accumulators, zero between launches */
     unsigned *counter;
+    const float *node;          /* node positions of the gate grid, index 0 at node -mom_n (rsc_nodes.cuh) */
+    float4 *stray;              /* the nodes' sums of single scatterers, zero between launches */
+    unsigned long long lead;    /* leading scatterers in spatial order */
     unsigned long long *runs;   /* the grouped compensated pulse's run counter, zero between launches (or null) */
     float4 *pulse;
     double *pulse64;
@@ -810,6 +813,8 @@ __global__ void k_eval_math(int fn, const float *a, const float *b, float *out, 
             out[i] = range_weight_tri(rwd, a[i]);
             break;
         }
+        case 13: out[i] = sqrt_mid(a[i]); break;
+        case 14: out[i] = div_by(a[i], b[i], rcp_mid(b[i])); break;
         default: out[i] = 0.0f; break;
     }
 }

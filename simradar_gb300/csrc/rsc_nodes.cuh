@@ -1,0 +1,449 @@
+/*
+ * rsc_nodes.cuh -- pulse formation on the triangle range weight, summed on
+ * the nodes of the gate grid.
+ *
+ * The triangle whose half width is a whole number n of gate spacings is
+ * linear in range between neighbouring gate origins: the weight a scatterer
+ * has in gate k is the interpolation, between the two nodes E_m <= r < E_m+1
+ * it lies between, of the weights W(k, m) of gate k at the nodes.  So a
+ * scatterer adds its signal to two nodes with the weights (E_m+1 - r) and
+ * (r - E_m) over the spacing, both exact differences times one reciprocal,
+ * and the last block forms every gate from its 2 n - 1 nodes.  The work per
+ * scatterer does not depend on n: a pulse sampled finely in range costs what
+ * a coarse one does.  The nodes are the gate origins the reference's running
+ * sum gives (rs.cl:1214), continued evenly on both sides.
+ *
+ * Each warp takes a contiguous piece of the state, 64 neighbours at a time,
+ * lane l holding scatterers l and l + 32.  A state in spatial order keeps a
+ * run within two neighbouring intervals, so the warp holds the sums of their
+ * three nodes in registers, lane by lane, and reduces them across its lanes
+ * only when a run leaves them.
+ *
+ * What bounds it: the issue of its instructions.  README scale (2,001,920
+ * scatterers, 40 gates, n = 2): 13.0 M warp instructions, 24.9 us alone,
+ * against 22.0 M and 35.0 us for the sums gate by gate (k_pulse_group); the
+ * step beside the advance 67.1 -> 57.6 us.  500,000 scatterers on 240 gates
+ * (n = 12, which the gate window did not hold: every gate visited) 441 ->
+ * 19 us.  The signal's quotients and roots share one range check per
+ * scatterer instead of one each.  Written on packed pairs instead of two
+ * scalar scatterers it issued 10% fewer instructions (each constant of a
+ * packed operation costs its moves) but needed 77-104 registers and was
+ * slower (26.9 us); runs staged in shared memory by cp.async (the addresses
+ * and the copies' own loads cost more than the latency they hid) 31.0.
+ */
+#ifndef SIMRADAR_GB300_RSC_NODES_CUH
+#define SIMRADAR_GB300_RSC_NODES_CUH
+
+#include "rsc_pulse.cuh"
+
+namespace rsc {
+
+/* Largest half width of the triangle, in gate spacings. */
+constexpr int kNodeMaxN = 64;
+
+/* A scatterer's signal: its range, and signal x angular weight of each lane
+ * (Ih, Qh, Iv, Qv). */
+struct Sig {
+    float r, s[4];
+};
+
+/* signal_plain.  The range, the phase and the angular weight are its values
+ * bit for bit (rsc_mid.cuh; the three direction cosines share one reciprocal);
+ * 1 / r^2 is taken of the squared range and joins the angular weight before
+ * the rotation, whose sums are fused.  False when a scatterer is beyond 60
+ * degrees off the beam, closer than 2^-30 m or at a phase above 6e6 rad: the
+ * caller takes signal_plain. */
+__device__ __forceinline__ bool signal_plain_mid(const PulseArgs &P, const float4 &p, const float4 &x, Sig &o) {
+    const float *sd = P.sim;
+    const float s = p.x * p.x + p.y * p.y + p.z * p.z;
+    const float r = sqrt_mid(s);
+    /* the cosine of the beam angle, each direction cosine rounded */
+    const float y = rcp_mid(r);
+    const float dot = sd[0] * div_by(p.x, r, y) + sd[1] * div_by(p.y, r, y) + sd[2] * div_by(p.z, r, y);
+    const float phase = r * sd[4];
+    /* 1 / r^2, as the reciprocal of the squared range */
+    float k = rcp_mid(s);
+    /* acos(dot) = 2 asin(sqrt((1 - dot) / 2)), 0 past 1 (rsm_acosf); the
+     * doubling joins the table's scale, which is exact */
+    const float z = fmaxf(fmaf(dot, -0.5f, 0.5f), 0.0f);
+    const float sz = sqrt_from(z, rsqrt_approx(fmaxf(z, 0x1p-80f)));
+    const float half = fmaf(sz * z, rsm_asin_poly(z), sz), scale = 2.0f * P.awd[0];
+    const float raw0 = cl_clamp(fmaf(half, scale, P.awd[1] + 0.0f), 0.0f, P.awd[2]);
+    const float raw1 = cl_clamp(fmaf(half, scale, P.awd[1] + 1.0f), 0.0f, P.awd[2]);
+    k = k * cl_mix(__ldg(P.aw + (uint32_t)raw0), __ldg(P.aw + (uint32_t)raw1), raw0 - floorf(raw0));
+    /* sine and cosine (rsm_sincosf): adding 1.5 x 2^23 rounds to the integer,
+     * whose low bits are then the sum's */
+    const float qm = __fadd_rn(phase * RSM_TWO_OVER_PI, 12582912.0f);
+    const float q = qm - 12582912.0f;
+    float t = fmaf(-q, RSM_PIO2_1, phase);
+    t = fmaf(-q, RSM_PIO2_2, t);
+    t = fmaf(-q, RSM_PIO2_3, t);
+    float ss, cc;
+    {
+        const float w = t * t;
+        float ps = fmaf(0x1.71de3ap-19f, w, -0x1.a01a02p-13f);   /* rsm_sincos_reduced */
+        ps = fmaf(ps, w, 0x1.111112p-7f);
+        ps = fmaf(ps, w, -0x1.555556p-3f);
+        const float sn = fmaf(t * w, ps, t);
+        float pc = fmaf(-0x1.27e4fcp-22f, w, 0x1.a01a02p-16f);
+        pc = fmaf(pc, w, -0x1.6c16c2p-10f);
+        pc = fmaf(pc, w, 0x1.555556p-5f);
+        pc = fmaf(pc, w, -0.5f);
+        const float cs = fmaf(w, pc, 1.0f);
+        const unsigned b = __float_as_uint(qm);
+        const bool swap = (b & 1u) != 0u;
+        ss = __uint_as_float(__float_as_uint(swap ? cs : sn) ^ ((b & 2u) << 30)) * k;
+        cc = __uint_as_float(__float_as_uint(swap ? sn : cs) ^ (((b + 1u) & 2u) << 30)) * k;
+    }
+    o.r = r;
+    o.s[0] = fmaf(x.x, cc, x.y * ss);
+    o.s[1] = fmaf(x.y, cc, -(x.x * ss));
+    o.s[2] = fmaf(x.z, cc, x.w * ss);
+    o.s[3] = fmaf(x.w, cc, -(x.z * ss));
+    return dot > 0.5f && dot <= 0x1.00002p+0f && s > 0x1p-60f && fabsf(phase) < 6.0e6f;
+}
+
+/* The sum of four values over the warp's lanes: the sum of value c in lanes
+ * 8 c .. 8 c + 7 (six shuffles). */
+__device__ __forceinline__ float warp_sum4(unsigned lane, float v0, float v1, float v2, float v3) {
+    const bool h16 = (lane & 16u) != 0;
+    float k0 = h16 ? v2 : v0, k1 = h16 ? v3 : v1;
+    k0 = k0 + __shfl_xor_sync(0xffffffffu, h16 ? v0 : v2, 16);
+    k1 = k1 + __shfl_xor_sync(0xffffffffu, h16 ? v1 : v3, 16);
+    const bool h8 = (lane & 8u) != 0;
+    float k = h8 ? k1 : k0;
+    k = k + __shfl_xor_sync(0xffffffffu, h8 ? k0 : k1, 8);
+    k = k + __shfl_xor_sync(0xffffffffu, k, 4);
+    k = k + __shfl_xor_sync(0xffffffffu, k, 2);
+    return k + __shfl_xor_sync(0xffffffffu, k, 1);
+}
+
+/* Nodes of a pulse of G gates: m = -n .. G + n - 1, at index m + n. */
+__host__ __device__ __forceinline__ unsigned node_count(unsigned G, int n) { return G + 2u * (unsigned)n; }
+__host__ __device__ __forceinline__ size_t node_smem_bytes(unsigned G, int n) {
+    return (size_t)node_count(G, n) * 4 * sizeof(double);
+}
+
+/* 4 blocks of 256 per SM at 64 registers, nothing spilled.  README scale,
+ * pulse alone: 24.9 us; 26.9 with 3 blocks at 77 registers, 24.8 with 2 of
+ * 512, 28.1 with 8 of 128. */
+constexpr int kNodeThreads = 256, kNodeMinBlocks = 4;
+
+/* Runs a warp should have at least: a small state takes fewer blocks
+ * (131,072 scatterers, pulses read back: 17.8 us per step with 1, 18.3 with
+ * 2, 21.3 with 3). */
+constexpr unsigned kNodeRuns = 1;
+
+/* Copies of the nodes' sums that single scatterers are added to (a power of
+ * two): blocks share a copy, so that few meet in an address. */
+constexpr unsigned kNodeCopies = 8;
+__host__ __device__ __forceinline__ unsigned node_copies(unsigned G, int n) {
+    unsigned c = kNodeCopies;
+    while (c > 1 && c * node_count(G, n) > 1024u) c >>= 1;
+    return c;
+}
+
+/* Scatterers of a run that make a window worth moving to them (a move costs a
+ * reduction of its sums, about what eight scatterers alone cost). */
+constexpr int kNodePart = 8;
+/* ... and that let the others go one by one without looking for a window. */
+constexpr int kNodeMost = 40;
+
+/* A warp's window of three nodes and their sums, lane by lane (plain form). */
+struct NodeWindow {
+    float E0, E1, E2, i0, i1;
+    int c;              /* node index of E0, -1: none yet */
+    float acc[3][4];
+
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+#pragma unroll
+            for (int l = 0; l < 4; l++) acc[m][l] = 0.0f;
+        }
+    }
+    __device__ __forceinline__ void move(const PulseArgs &P, int node) {
+        c = node;
+        E0 = __ldg(P.node + node);
+        E1 = __ldg(P.node + node + 1);
+        E2 = __ldg(P.node + node + 2);
+        i0 = 1.0f / (E1 - E0);
+        i1 = 1.0f / (E2 - E1);
+        clear();
+    }
+    __device__ __forceinline__ bool holds(float r) const { return r >= E0 && r < E2; }
+    /* a scatterer at a range in [E0, E2) weighed onto the three nodes */
+    __device__ __forceinline__ void add(const Sig &g) {
+        const float w0 = fmaxf((E1 - g.r) * i0, 0.0f);
+        const float w1 = fminf((g.r - E0) * i0, (E2 - g.r) * i1);
+        const float w2 = fmaxf((g.r - E1) * i1, 0.0f);
+        fma_pair(w0, g.s[0], g.s[1], acc[0][0], acc[0][1]);
+        fma_pair(w0, g.s[2], g.s[3], acc[0][2], acc[0][3]);
+        fma_pair(w1, g.s[0], g.s[1], acc[1][0], acc[1][1]);
+        fma_pair(w1, g.s[2], g.s[3], acc[1][2], acc[1][3]);
+        fma_pair(w2, g.s[0], g.s[1], acc[2][0], acc[2][1]);
+        fma_pair(w2, g.s[2], g.s[3], acc[2][2], acc[2][3]);
+    }
+    /* the lanes' sums into the block's bins */
+    __device__ __forceinline__ void flush(double *bins, unsigned lane) {
+        if (c < 0) return;
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            const float k = warp_sum4(lane, acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
+            if ((lane & 7u) == 0u && k != 0.0f) atomicAdd(bins + 4 * (c + m) + (lane >> 3), (double)k);
+        }
+        c = -1;
+    }
+};
+
+/* A scatterer with a non-finite signal reaches every gate, its weight there
+ * as pass 1 forms it (0 x NaN is NaN): straight into the grid's sums of the
+ * gates, which the last block adds to what the nodes give. */
+__device__ __noinline__ void node_non_finite(const PulseArgs &P, float r, float v0, float v1, float v2, float v3) {
+    double *gate = P.acc64 + 4 * (size_t)node_count(P.G, P.mom_n);
+    for (unsigned k = 0; k < P.G; k++) {
+        const float w = range_weight(P, r - __ldg(P.rk + k));
+        atomicAdd(gate + 4 * k + 0, (double)(w * v0));
+        atomicAdd(gate + 4 * k + 1, (double)(w * v1));
+        atomicAdd(gate + 4 * k + 2, (double)(w * v2));
+        atomicAdd(gate + 4 * k + 3, (double)(w * v3));
+    }
+}
+
+/* Index of the interval [E_j, E_j+1) that holds r, -1 outside the nodes. */
+__device__ __forceinline__ int node_interval(const PulseArgs &P, float r) {
+    const int last = (int)node_count(P.G, P.mom_n) - 2;
+    const float jf = floorf((r - __ldg(P.node)) * P.inv_delta);
+    if (!(jf >= -1.0f && jf <= (float)(last + 1))) return -1;
+    int j = min(max((int)jf, 0), last);
+    /* the quotient can be one off beside a node */
+    if (r < __ldg(P.node + j)) j--;
+    else if (r >= __ldg(P.node + j + 1)) j++;
+    return j > last ? -1 : j;
+}
+
+/* One scatterer, in interval j, by itself: two 16-byte reductions in L2,
+ * which nothing waits for. */
+__device__ __forceinline__ void red_add4(float4 *p, float a, float b, float c, float d) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ void node_stray(const PulseArgs &P, float4 *stray, int j, float r, const float *v) {
+    const float a = __ldg(P.node + j), b = __ldg(P.node + j + 1), i = 1.0f / (b - a);
+    const float wa = (b - r) * i, wb = (r - a) * i;
+    red_add4(stray + j, wa * v[0], wa * v[1], wa * v[2], wa * v[3]);
+    red_add4(stray + j + 1, wb * v[0], wb * v[1], wb * v[2], wb * v[3]);
+}
+
+/* A lane's scatterer by itself: to every gate when not finite, nowhere when
+ * it reaches none. */
+__device__ __forceinline__ bool sig_finite(const Sig &g) { return fabsf(g.r) < INFINITY && finite4(g.s); }
+__device__ __forceinline__ void node_alone(const PulseArgs &P, const Sig &g, float4 *stray) {
+    if (!sig_finite(g)) {
+        node_non_finite(P, g.r, g.s[0], g.s[1], g.s[2], g.s[3]);
+        return;
+    }
+    const int j = node_interval(P, g.r);
+    if (j >= 0) node_stray(P, stray, j, g.r, g.s);
+}
+
+/* A run the window holds little of.  Scatterers that reach no gate drop out
+ * and non-finite ones go to every gate; what the window, or one moved to
+ * where a good part of the run lies, holds is added to it, and the rest --
+ * debris, scatterers respawned elsewhere since the last sort -- one by one. */
+__device__ __forceinline__ void node_settle(const PulseArgs &P, NodeWindow &W, const Sig *g, unsigned in, double *bins,
+                                            float4 *stray, unsigned lane) {
+    int j[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        j[q] = -1;
+        if (!((in >> q) & 1u)) continue;
+        if (!sig_finite(g[q])) {
+            node_non_finite(P, g[q].r, g[q].s[0], g[q].s[1], g[q].s[2], g[q].s[3]);
+        } else {
+            j[q] = node_interval(P, g[q].r);
+        }
+    }
+    for (;;) {
+        const unsigned l0 = __ballot_sync(0xffffffffu, j[0] >= 0), l1 = __ballot_sync(0xffffffffu, j[1] >= 0);
+        if ((l0 | l1) == 0u) return;
+        const auto within = [&](int c) {
+            return __popc(__ballot_sync(0xffffffffu, j[0] >= 0 && (unsigned)(j[0] - c) < 2u)) +
+                   __popc(__ballot_sync(0xffffffffu, j[1] >= 0 && (unsigned)(j[1] - c) < 2u));
+        };
+        if (W.c < 0 || within(W.c) < kNodePart) {
+            /* where a few of those left lie: any of them may be astray */
+            int best = 0, at = 0;
+            unsigned t0 = l0, t1 = l1;
+#pragma unroll 1
+            for (int t = 0; t < 4 && best < kNodePart && (t0 | t1) != 0u; t++) {
+                const int src = __ffs(t0 ? t0 : t1) - 1;
+                const int cand = __shfl_sync(0xffffffffu, t0 ? j[0] : j[1], src);
+                const int a = within(cand - 1), b = within(cand);
+                best = max(a, b);
+                at = a > b ? cand - 1 : cand;
+                /* the next a quarter of the run on */
+                if (t0) t0 &= ~(0x1ffu << (src & ~7));
+                else t1 &= ~(0x1ffu << (src & ~7));
+            }
+            if (best < kNodePart) {
+                if (j[0] >= 0) node_stray(P, stray, j[0], g[0].r, g[0].s);
+                if (j[1] >= 0) node_stray(P, stray, j[1], g[1].r, g[1].s);
+                return;
+            }
+            W.flush(bins, lane);
+            W.move(P, min(max(at, 0), (int)node_count(P.G, P.mom_n) - 3));
+        }
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            if (j[q] >= 0 && (unsigned)(j[q] - W.c) < 2u) {
+                W.add(g[q]);
+                j[q] = -1;
+            }
+        }
+    }
+}
+
+/* The block's node sums into the grid's accumulator, the last block forming
+ * the gates and leaving accumulator and counter at zero. */
+__device__ __forceinline__ void node_finish(const PulseArgs &P, double *bins, unsigned nblk) {
+    const unsigned nodes = node_count(P.G, P.mom_n), outs = P.G * 4;
+    __syncthreads();
+    for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) {
+        const double v = bins[o];
+        if (v != 0.0) atomicAdd(P.acc64 + o, v);
+    }
+    __shared__ bool s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        /* after the barrier this fence orders every thread's reductions */
+        __threadfence();
+        s_last = atomicAdd(P.counter, 1u) == nblk - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+    float *sums = reinterpret_cast<float *>(bins), *at_node = sums + 4 * nodes;
+    const unsigned copies = node_copies(P.G, P.mom_n);
+    const float *stray = reinterpret_cast<const float *>(P.stray);
+    /* the loads of several sums in flight at once: no store between them */
+#pragma unroll 4
+    for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) {
+        float v = (float)__ldcg(P.acc64 + o), t = 0.0f;
+#pragma unroll
+        for (unsigned c = 0; c < kNodeCopies; c++) {
+            if (c < copies) t = t + __ldcg(stray + (size_t)c * 4 * nodes + o);
+        }
+        sums[o] = v + t;   /* over bins[o / 2], whose sums are out */
+    }
+    for (unsigned o = threadIdx.x; o < nodes; o += blockDim.x) at_node[o] = __ldg(P.node + o);
+    __syncthreads();
+    for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) P.acc64[o] = 0.0;
+    for (unsigned o = threadIdx.x; o < nodes * copies; o += blockDim.x) P.stray[o] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int n = P.mom_n;
+    for (unsigned o = threadIdx.x; o < outs; o += blockDim.x) {
+        const unsigned k = o >> 2, l = o & 3u;
+        const float rk = __ldg(P.rk + k);
+        float sum = 0.0f;
+        const unsigned end = min(k + 2u * (unsigned)n + 1u, nodes);
+#pragma unroll 4
+        for (unsigned at = k; at < end; at++) {
+            const float w = fmaxf(1.0f - fabsf(at_node[at] - rk) * P.rwd[0], 0.0f);
+            sum = fmaf(w, sums[4 * at + l], sum);
+        }
+        double *extra = P.acc64 + 4 * (size_t)nodes + o;
+        const double e = __ldcg(extra);
+        if (e != 0.0) {
+            sum = (float)((double)sum + e);
+            *extra = 0.0;
+        }
+        reinterpret_cast<float *>(P.pulse)[o] = sum;
+    }
+    if (threadIdx.x == 0) *P.counter = 0u;
+}
+
+__device__ __forceinline__ void node_body(const PulseArgs &P, unsigned blk, unsigned nblk) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *bins = reinterpret_cast<double *>(smem_raw);
+    const unsigned nodes = node_count(P.G, P.mom_n);
+    float4 *stray = P.stray + (size_t)nodes * (blk & (node_copies(P.G, P.mom_n) - 1u));
+    for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) bins[o] = 0.0;
+    __syncthreads();
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned long long n = P.n, runs = (n + 63ull) / 64ull, whole = n / 64ull;
+    const unsigned long long warps = (unsigned long long)nblk * (blockDim.x >> 5);
+    const unsigned long long me = (unsigned long long)blk * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    /* a contiguous piece of the runs in spatial order, and every warps-th of
+     * the others, which cost more each */
+    const unsigned long long lead = P.lead / 64ull;
+    const unsigned long long last = lead * (me + 1) / warps;
+    NodeWindow W;
+    W.c = -1;
+    W.E0 = W.E1 = W.E2 = NAN;
+    W.i0 = W.i1 = 0.0f;
+    W.clear();
+    const auto next = [&](unsigned long long r) {
+        r++;
+        return r == last ? lead + me : (r > last ? r + (warps - 1) : r);
+    };
+    unsigned long long run = lead * me / warps;
+    if (run == last) run = lead + me;
+    for (; run < runs; run = next(run)) {
+        const float4 *pp = P.pos + run * 64ull + lane, *xx = P.rcs + run * 64ull + lane;
+        float4 p[2], x[2];
+        unsigned in = 3u;
+        if (run < whole) {
+            p[0] = __ldg(pp);
+            p[1] = __ldg(pp + 32);
+            x[0] = __ldg(xx);
+            x[1] = __ldg(xx + 32);
+        } else {
+            /* past the end: the last scatterer with no backscatter */
+            const unsigned left = (unsigned)(n - run * 64ull);
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const bool past = lane + 32u * q >= left;
+                p[q] = __ldg(past ? P.pos + (n - 1) : pp + 32 * q);
+                x[q] = past ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : __ldg(xx + 32 * q);
+                if (past) in &= ~(1u << q);
+            }
+        }
+        Sig g[2];
+        bool held[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            if (!signal_plain_mid(P, p[q], x[q], g[q])) {
+                Sig32 sg;
+                signal_plain(P, p[q], x[q], sg);
+                g[q].r = sg.r;
+#pragma unroll
+                for (int l = 0; l < 4; l++) g[q].s[l] = sg.s.v[l];
+            }
+            /* NaN or an infinity in any lane makes the sum NaN */
+            const float f = fmaf(g[q].s[0], 0.0f, fmaf(g[q].s[1], 0.0f, fmaf(g[q].s[2], 0.0f, g[q].s[3] * 0.0f)));
+            held[q] = W.holds(g[q].r) && f == 0.0f;
+        }
+        if (__all_sync(0xffffffffu, held[0] && held[1])) {
+            W.add(g[0]);
+            W.add(g[1]);
+        } else if (__popc(__ballot_sync(0xffffffffu, held[0])) + __popc(__ballot_sync(0xffffffffu, held[1])) >=
+                   kNodeMost) {
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                if (held[q]) W.add(g[q]);
+                else if ((in >> q) & 1u) node_alone(P, g[q], stray);
+            }
+        } else {
+            node_settle(P, W, g, in, bins, stray, lane);
+        }
+    }
+    W.flush(bins, lane);
+    node_finish(P, bins, nblk);
+}
+
+__global__ void __launch_bounds__(kNodeThreads, kNodeMinBlocks) k_pulse_nodes(const PulseArgs P) {
+    node_body(P, blockIdx.x, gridDim.x);
+}
+
+}  // namespace rsc
+
+#endif

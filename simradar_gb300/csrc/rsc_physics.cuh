@@ -15,6 +15,7 @@
 #include <stdint.h>
 
 #include "rsmath.h"
+#include "rsc_mid.cuh"
 
 namespace rsc {
 
