@@ -99,6 +99,7 @@ struct rsc_worker {
     float *angular_weight = nullptr;
     uint32_t angular_n = 0;
     float angular_desc[4] = {0};
+    bool angular_finite = true;
     float4 *ellipsoid = nullptr;
     uint32_t ellipsoid_n = 0;
     float ellipsoid_desc[4] = {0};
@@ -466,6 +467,7 @@ PulseKernel pulse_kernel(int mode, int path) {
         return path == 2 ? rsc::k_pulse<0, 2> : (path == 1 ? rsc::k_pulse<0, 1> : rsc::k_pulse<0, 0>);
     }
     if (mode == RSC_PULSE_COMPENSATED) {
+        if (path == 5) return rsc::k_pulse_nodes_comp;
         if (path == 4) return rsc::k_pulse_group<1, kPulseGroup, 1>;
         return path == 3 ? rsc::k_pulse_group<1, kPulseGroup> : rsc::k_pulse<1, -1>;
     }
@@ -477,7 +479,7 @@ PulseKernel pulse_kernel(int mode, int path) {
  * when it does not write aux / sig), 4 the same with the triangle range
  * table compiled in */
 int pulse_path(const PulseArgs &P, int mode) {
-    if (mode == RSC_PULSE_PLAIN && P.mom_n > 0) return 5;
+    if (mode != RSC_PULSE_F64 && P.mom_n > 0) return 5;
     if (P.dense) return 2;
     if (P.coherent_span <= 0) return 0;
     if ((mode == RSC_PULSE_PLAIN && !P.materialize) || mode == RSC_PULSE_COMPENSATED) return P.rw_tri ? 4 : 3;
@@ -498,10 +500,12 @@ int pulse_shape(int mode, bool batch, uint32_t G, int want_warps, int want_per_s
     if (path == 5) {
         const int warps = rsc::kNodeThreads / 32;
         *threads = 32 * (want_warps > 0 && want_warps < warps ? want_warps : warps);
-        *smem = rsc::node_smem_bytes(G, mom_n);
+        *smem = rsc::node_smem_bytes(G, mom_n, mode == RSC_PULSE_COMPENSATED);
         int fit = 1;
-        cudaError_t e = batch ? kernel_occupancy(rsc::k_pulse_batch_nodes, *threads, *smem, &fit)
-                              : kernel_occupancy(pulse_kernel(mode, path), *threads, *smem, &fit);
+        cudaError_t e = !batch ? kernel_occupancy(pulse_kernel(mode, path), *threads, *smem, &fit)
+                        : mode == RSC_PULSE_PLAIN
+                            ? kernel_occupancy(rsc::k_pulse_batch_nodes<0>, *threads, *smem, &fit)
+                            : kernel_occupancy(rsc::k_pulse_batch_nodes<1>, *threads, *smem, &fit);
         if (e != cudaSuccess) return cuda_fail(RSC_ERR_CUDA, "pulse kernel configuration: %s", cudaGetErrorString(e));
         if (want_per_sm <= 0) want_per_sm = kNodePerSm;
         if (fit < 1) fit = 1;
@@ -661,15 +665,22 @@ double window_margin(double drift, float range_start, float range_delta, uint32_
     return (drift + 2.0 * ulp_r) / delta + 8.0 * ldexp(1.0, -23) * span + 1.0e-4;
 }
 
-/* The plain pulse through the node sums where the triangle allows them: a
- * state in spatial order, or a triangle too wide for the gate window. */
-void use_nodes(rsc_worker *w, PulseArgs &P) {
+/* A pulse through the node sums where the triangle allows them: compensated
+ * always (unless rsc_set_pulse_moments turned them off), plain on a state in
+ * spatial order or with a triangle too wide for the gate window. */
+void use_nodes(rsc_worker *w, PulseArgs &P, int mode) {
     const int n = node_span(P);
-    if (n == 0 || (P.coherent_span <= 0 && !P.dense)) return;
+    if (mode == RSC_PULSE_PLAIN ? n == 0 || (P.coherent_span <= 0 && !P.dense) : n == 0 || !w->moments) return;
     P.mom_n = n;
     P.node = w->node + (rsc::kNodeMaxN - n);
-    P.stray = reinterpret_cast<float4 *>(w->acc64 + (rsc::node_count(w->G, rsc::kNodeMaxN) + w->G) * 4);
+    P.stray = reinterpret_cast<float4 *>(w->acc64 + (2 * rsc::node_count(w->G, rsc::kNodeMaxN) + w->G) * 4);
     P.lead = w->perm != nullptr ? w->sort_end : 0;
+    /* half a gate more than the triangles reach; everything when an antenna
+     * weight is not finite, which any range meets */
+    const double lo = (double)w->range_start - (n + 0.5) * (double)w->range_delta;
+    const double hi = (double)w->range_start + (w->G - 1 + n + 0.5) * (double)w->range_delta;
+    P.reach_lo2 = lo > 0.0 && w->angular_finite ? (float)(lo * lo) : 0.0f;
+    P.reach_hi2 = hi > 0.0 && w->angular_finite ? (float)(hi * hi) : INFINITY;
 }
 
 void fill_pulse_args(rsc_worker *w, PulseArgs &P, const float *sim) {
@@ -688,7 +699,7 @@ void fill_pulse_args(rsc_worker *w, PulseArgs &P, const float *sim) {
     P.rk64 = w->rk64;
     P.G = w->G;
     memcpy(P.sim, sim, sizeof(P.sim));
-    rsc::beam_norm_df(P.sim, P.bn_hi, P.bn_lo);
+    rsc::beam_norm_df(P.sim, P);
     P.rs = w->range_start;
     P.inv_delta = w->range_delta != 0.0f ? 1.0f / w->range_delta : 0.0f;
     P.rdelta = w->range_delta;
@@ -875,9 +886,9 @@ int rsc_worker_malloc(rsc_worker *w, size_t num_scats, float range_start, float 
     RSC_CUDA(cudaMalloc((void **)&w->rk64, range_count * sizeof(double)));
     const size_t nodes = rsc::node_count(range_count, rsc::kNodeMaxN);
     RSC_CUDA(cudaMalloc((void **)&w->node, nodes * sizeof(float)));
-    /* the pulse kernels' FP64 accumulator (gates, or nodes and then gates);
+    /* the pulse kernels' FP64 accumulator (gates; or nodes, or intervals, and then gates);
      * each launch leaves it at zero */
-    const size_t acc_bytes = (nodes + range_count) * 4 * sizeof(double) + kStrayFloat4s * sizeof(float4);
+    const size_t acc_bytes = (2 * nodes + range_count) * 4 * sizeof(double) + kStrayFloat4s * sizeof(float4);
     RSC_CUDA(cudaMalloc((void **)&w->acc64, acc_bytes));
     RSC_CUDA(cudaMemsetAsync(w->acc64, 0, acc_bytes, w->stream));
     RSC_CUDA(cudaMalloc((void **)&w->counter, sizeof(unsigned)));
@@ -921,6 +932,8 @@ int rsc_set_angular_weight(rsc_worker *w, const float *table, uint32_t n, const 
     s = upload_floats(&w->angular_weight, table, n);
     if (s) return s;
     w->angular_n = n;
+    w->angular_finite = true;
+    for (uint32_t k = 0; k < n; k++) w->angular_finite = w->angular_finite && fabsf(table[k]) < INFINITY;
     memcpy(w->angular_desc, desc, sizeof(w->angular_desc));
     return RSC_OK;
 }
@@ -1683,12 +1696,11 @@ int rsc_make_pulse(rsc_worker *w, const float sim_desc[16]) {
         P.rk = w->rk_hi;
         /* the error-free warp sums need the grouped path, whatever the order */
         P.coherent_span = (int)w->G + 1;
-        P.mom_n = w->moments ? moment_span(P) : 0;
         P.runs = w->runs;
     }
     const bool mat = (mode == RSC_PULSE_PLAIN) && (w->materialize || sim_desc[15] != 0.0f);
     P.materialize = mat ? 1 : 0;
-    if (mode == RSC_PULSE_PLAIN && !mat && !w->pend) use_nodes(w, P);
+    if (mode != RSC_PULSE_F64 && !mat && !w->pend) use_nodes(w, P, mode);
     int grid = 0, threads = 0;
     size_t smem = 0;
     s = pulse_geometry(w, mode, pulse_path(P, mode), P.mom_n, &grid, &threads, &smem);
@@ -1702,7 +1714,6 @@ int rsc_make_pulse(rsc_worker *w, const float sim_desc[16]) {
         size_t ssmem = 0;
         s = step_shape(mode, w, &sgrid, &ssmem);
         if (s) return s;
-        P.mom_n = 0;   /* the fused kernel sums per gate */
         if (mode == RSC_PULSE_PLAIN) {
             rsc::k_step<0><<<sgrid, rsc::kAdvanceThreads, ssmem, w->stream>>>(w->pend_a, P, w->pend_blocks);
         } else {
@@ -1868,7 +1879,7 @@ struct rsc_batch {
      * (0: as many as fit) */
     int adv_threads = rsc::kAdvanceThreads, adv_per_sm = 0;
     size_t adv_smem = 0;
-    bool nodes = false; /* the plain pulse through the node sums */
+    bool nodes = false; /* the pulse through the node sums */
     bool tri = false;   /* the pulse kernel with the triangle range weight compiled in */
     /* per-instance launch descriptors and block prefixes */
     std::vector<rsc::BatchAdvance> h_adv;
@@ -1998,18 +2009,25 @@ int batch_prepare(rsc_batch *b, const rsc::BatchStep *row) {
         if (b->mode == RSC_PULSE_COMPENSATED) {
             P.rk = x->rk_hi;
             P.coherent_span = (int)x->G + 1;
-            P.mom_n = x->moments ? moment_span(P) : 0;
             P.runs = x->runs;
         }
         P.materialize = 0;
-        if (b->mode == RSC_PULSE_PLAIN) use_nodes(x, P);
+        if (b->mode != RSC_PULSE_F64 && !b->persist) use_nodes(x, P, b->mode);
         nodes = nodes && P.mom_n > 0;
         max_n = std::max(max_n, P.mom_n);
         tri = tri && P.rw_tri;
         b->concept[i] = rsm_f2u(row[i].sim[5]);
     }
-    /* the plain pulse through the node sums when every instance's may */
-    nodes = nodes && b->mode == RSC_PULSE_PLAIN;
+    /* through the node sums when every instance's pulse may */
+    nodes = nodes && b->mode != RSC_PULSE_F64 && !b->persist;
+    if (!nodes) {
+        /* the sums gate by gate, or their moments per interval */
+        for (size_t i = 0; i < n; i++) {
+            PulseArgs &P = b->h_pulse[i];
+            P.mom_n = b->mode == RSC_PULSE_COMPENSATED && b->w[i]->moments ? moment_span(P) : 0;
+        }
+        max_n = 0;
+    }
     s = pulse_shape(b->mode, true, b->Gmax, b->tune_warps, b->tune_per_sm, &per_sm, &threads, &smem, nodes ? 5 : 0, max_n);
     if (s) return s;
     const double total = (double)b->num_sms * per_sm;
@@ -2059,8 +2077,10 @@ cudaError_t batch_launch_pulse(rsc_batch *b, int k) {
     float4 *out = b->d_out + (size_t)k * n * b->Gmax;
     const unsigned g = b->pulse_blocks, t = (unsigned)b->pulse_threads;
     const size_t sm = b->pulse_smem;
-    if (b->nodes) {
-        rsc::k_pulse_batch_nodes<<<g, t, sm, b->stream>>>(b->d_pulse, st, b->d_pulse_prefix, n, out, b->Gmax);
+    if (b->nodes && b->mode == RSC_PULSE_COMPENSATED) {
+        rsc::k_pulse_batch_nodes<1><<<g, t, sm, b->stream>>>(b->d_pulse, st, b->d_pulse_prefix, n, out, b->Gmax);
+    } else if (b->nodes) {
+        rsc::k_pulse_batch_nodes<0><<<g, t, sm, b->stream>>>(b->d_pulse, st, b->d_pulse_prefix, n, out, b->Gmax);
     } else if (b->mode == RSC_PULSE_PLAIN && b->tri) {
         rsc::k_pulse_batch<0, 1><<<g, t, sm, b->stream>>>(b->d_pulse, st, b->d_pulse_prefix, n, out, b->Gmax);
     } else if (b->mode == RSC_PULSE_PLAIN) {
@@ -2295,11 +2315,10 @@ int rsc_autotune(rsc_worker *w, const float sim_desc[16], int *warps_out, int *b
     if (mode == RSC_PULSE_COMPENSATED) {
         P.rk = w->rk_hi;
         P.coherent_span = (int)w->G + 1;
-        P.mom_n = w->moments ? moment_span(P) : 0;
         P.runs = w->runs;
     }
     P.materialize = 0;
-    if (mode == RSC_PULSE_PLAIN) use_nodes(w, P);
+    if (mode != RSC_PULSE_F64) use_nodes(w, P, mode);
     s = pulse_d2h_wait(w);
     if (s) return s;
     EventPair ev;
@@ -3135,7 +3154,7 @@ int rsc_make_pulse_noalloc(const float *pos4, const float *rcs4, size_t num_scat
     P.rk = reinterpret_cast<const float *>(b + RSC_NA_RK_OFF);
     P.G = G;
     memcpy(P.sim, sim_desc, sizeof(P.sim));
-    rsc::beam_norm_df(P.sim, P.bn_hi, P.bn_lo);
+    rsc::beam_norm_df(P.sim, P);
     P.rs = range_start;
     P.inv_delta = range_delta != 0.0f ? 1.0f / range_delta : 0.0f;
     P.rdelta = range_delta;

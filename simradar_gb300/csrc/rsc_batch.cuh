@@ -146,21 +146,22 @@ __device__ __forceinline__ int batch_pulse_args(PulseArgs &sp, int &s_i, const P
         sp.pulse = out + (size_t)i * out_stride;
         sp.pos = steps[i].pos_r;
         sp.rcs = steps[i].rcs_r;
-        beam_norm_df(steps[i].sim, sp.bn_hi, sp.bn_lo);
+        beam_norm_df(steps[i].sim, sp);
     }
     __syncthreads();
     return i;
 }
 
-/* Every instance's plain pulse through its node sums (rsc_nodes.cuh). */
-__global__ void __launch_bounds__(kNodeThreads, kNodeMinBlocks)
+/* Every instance's pulse through its node sums (rsc_nodes.cuh). */
+template <int MODE>
+__global__ void __launch_bounds__(kNodeThreads, MODE == 0 ? kNodeMinBlocks : kCompMinBlocks)
 k_pulse_batch_nodes(const PulseArgs *inst, const BatchStep *steps, const unsigned *prefix, int ninst, float4 *out,
                     unsigned out_stride) {
     __shared__ __align__(16) PulseArgs sp;
     __shared__ int s_i;
     const int i = batch_pulse_args(sp, s_i, inst, steps, prefix, ninst, out, out_stride);
     const unsigned b0 = __ldg(prefix + i);
-    node_body(sp, blockIdx.x - b0, __ldg(prefix + i + 1) - b0);
+    node_body<MODE>(sp, blockIdx.x - b0, __ldg(prefix + i + 1) - b0);
 }
 
 /* TRI 1: every instance's range table is the triangle (compiled in) */
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(kPersistThreads, 4) k_batch_persist(const Pers
                 sp.counter = A.tick + slot;
                 sp.pos = st->pos_r;
                 sp.rcs = st->rcs_r;
-                beam_norm_df(st->sim, sp.bn_hi, sp.bn_lo);
+                beam_norm_df(st->sim, sp);
             }
             __syncthreads();
             persist_pulse<MODE, TRI>(sp, start, end, __ldg(A.nblk + i));

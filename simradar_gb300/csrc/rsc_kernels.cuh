@@ -467,6 +467,7 @@ struct PulseArgs {
     unsigned G;
     float sim[16];
     float bn_hi, bn_lo;  /* |beam| of sim[0..2] as a double-float (compensated form) */
+    float ib2_hi, ib2_lo;   /* and 1 / |beam|^2 */
     float rs, inv_delta, win_lo, win_hi;
     float rdelta;        /* gate spacing: the running sum's increment */
     unsigned rw_n;       /* range weight table length; <= 4 is kept in rwv */
@@ -481,6 +482,7 @@ struct PulseArgs {
     unsigned *counter;
     const float *node;          /* node positions of the gate grid, index 0 at node -mom_n (rsc_nodes.cuh) */
     float4 *stray;              /* the nodes' sums of single scatterers, zero between launches */
+    float reach_lo2, reach_hi2; /* squared ranges between which a scatterer can reach a gate, with a margin */
     unsigned long long lead;    /* leading scatterers in spatial order */
     unsigned long long *runs;   /* the grouped compensated pulse's run counter, zero between launches (or null) */
     float4 *pulse;
@@ -489,11 +491,13 @@ struct PulseArgs {
 
 /* The norm of the beam vector sim[0..2] as a double-float, formed once per
  * pulse in double (the compensated signal divides by |b| |p|). */
-__host__ __device__ inline void beam_norm_df(const float *sim, float &hi, float &lo) {
+__host__ __device__ inline void beam_norm_df(const float *sim, PulseArgs &P) {
     const double x = sim[0], y = sim[1], z = sim[2];
-    const double n = sqrt(x * x + y * y + z * z);
-    hi = (float)n;
-    lo = (float)(n - (double)hi);
+    const double n2 = x * x + y * y + z * z, n = sqrt(n2), i = 1.0 / n2;
+    P.bn_hi = (float)n;
+    P.bn_lo = (float)(n - (double)P.bn_hi);
+    P.ib2_hi = (float)i;
+    P.ib2_lo = (float)(i - (double)P.ib2_hi);
 }
 
 /* the pass-1 weight of one gate (rs.cl:1196-1209), bit-exact.  The clamp

@@ -120,14 +120,19 @@ __device__ __forceinline__ float warp_sum4(unsigned lane, float v0, float v1, fl
 
 /* Nodes of a pulse of G gates: m = -n .. G + n - 1, at index m + n. */
 __host__ __device__ __forceinline__ unsigned node_count(unsigned G, int n) { return G + 2u * (unsigned)n; }
-__host__ __device__ __forceinline__ size_t node_smem_bytes(unsigned G, int n) {
-    return (size_t)node_count(G, n) * 4 * sizeof(double);
+__host__ __device__ __forceinline__ size_t node_smem_bytes(unsigned G, int n, bool compensated) {
+    return (size_t)node_count(G, n) * (compensated ? 8 : 4) * sizeof(double);
 }
 
 /* 4 blocks of 256 per SM at 64 registers, nothing spilled.  README scale,
  * pulse alone: 24.9 us; 26.9 with 3 blocks at 77 registers, 24.8 with 2 of
  * 512, 28.1 with 8 of 128. */
 constexpr int kNodeThreads = 256, kNodeMinBlocks = 4;
+
+/* The compensated form: 3 blocks at 80 registers (40 bytes spilled) against 2
+ * at 115: a dwell of 3 pulses of 8.4 M scatterers 919 us against 941, of 2 of
+ * 33.7 M 3449 against 3486. */
+constexpr int kCompMinBlocks = 3;
 
 /* Runs a warp should have at least: a small state takes fewer blocks
  * (131,072 scatterers, pulses read back: 17.8 us per step with 1, 18.3 with
@@ -146,7 +151,11 @@ __host__ __device__ __forceinline__ unsigned node_copies(unsigned G, int n) {
 /* Scatterers of a run that make a window worth moving to them (a move costs a
  * reduction of its sums, about what eight scatterers alone cost). */
 constexpr int kNodePart = 8;
-/* ... and that let the others go one by one without looking for a window. */
+/* ... in runs of their own piece.  The other runs (sparse debris: a run spans
+ * several intervals; a state in the caller's order) move it for no fewer than
+ * this, and a run with as many in the window lets the rest go one by one
+ * without looking further (60,000 drops and 3 x 800 debris: 161 us for 8
+ * steps against 175 when sparse runs were taken window by window). */
 constexpr int kNodeMost = 40;
 
 /* A warp's window of three nodes and their sums, lane by lane (plain form). */
@@ -195,6 +204,238 @@ struct NodeWindow {
         c = -1;
     }
 };
+
+/* ---- the compensated form ----
+ * The same walk over the state with double-float sums.  Bound by instruction
+ * issue (FP32 adds and FMAs of the double-floats): README scale 36.6 M warp
+ * instructions and 59.6 us alone, against 61.9 M and 88.4 us for moments per
+ * interval reduced across the warp for every run of 64 with signal_comp's
+ * terms; 8.4 M scatterers at 30 km 266 -> 202 us; 77,777 on gates 7.5 m apart
+ * (too many for the gate window: every gate visited) 119 -> 15 us.  A gate's
+ * error against FP64 is what it was (rms 8.4e-9 of the sum of |x| on a
+ * 21,536-scatterer scene, both forms: the output's rounding). */
+
+/* Add the double-float (h, l) to the double-float sum (S, s). */
+__device__ __forceinline__ void df_acc(float &S, float &s, float h, float l) {
+    float a, e;
+    two_sum(S, h, a, e);
+    S = a;
+    s = s + (e + l);
+}
+
+/* The sum of four double-floats over the warp's lanes, the sum of value c in
+ * lanes 8 c .. 8 c + 7, heads added error-free. */
+__device__ __forceinline__ void warp_sum4_df(unsigned lane, const float *v, const float *u, float &S, float &s) {
+    const bool h16 = (lane & 16u) != 0, h8 = (lane & 8u) != 0;
+    float k0 = h16 ? v[2] : v[0], k1 = h16 ? v[3] : v[1], t0 = h16 ? u[2] : u[0], t1 = h16 ? u[3] : u[1];
+    df_acc(k0, t0, __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16),
+           __shfl_xor_sync(0xffffffffu, h16 ? u[0] : u[2], 16));
+    df_acc(k1, t1, __shfl_xor_sync(0xffffffffu, h16 ? v[1] : v[3], 16),
+           __shfl_xor_sync(0xffffffffu, h16 ? u[1] : u[3], 16));
+    S = h8 ? k1 : k0;
+    s = h8 ? t1 : t0;
+    df_acc(S, s, __shfl_xor_sync(0xffffffffu, h8 ? k0 : k1, 8), __shfl_xor_sync(0xffffffffu, h8 ? t0 : t1, 8));
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1)
+        df_acc(S, s, __shfl_xor_sync(0xffffffffu, S, off), __shfl_xor_sync(0xffffffffu, s, off));
+}
+
+/* Node j of the even grid, rs + (j - n) delta, as a double-float. */
+__device__ __forceinline__ void comp_node(const PulseArgs &P, int j, float &h, float &l) {
+    float a, b, s, e;
+    two_prod((float)(j - P.mom_n), P.rdelta, a, b);
+    two_sum(P.rs, a, s, e);
+    fast_two_sum(s, e + b, h, l);
+}
+
+/* f as a double by its bits: the FP64 units' conversions issue at 1/64 of the
+ * FP32 rate.  Values below 2^-126 count as 0. */
+__device__ __forceinline__ double wide_of(float f) {
+    const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
+    const unsigned hi = (m >> 3) + 0x38000000u, lo = b << 29;
+    return m < 0x00800000u ? 0.0 : __hiloint2double((int)(hi | (b & 0x80000000u)), (int)lo);
+}
+/* A double-float into a sum in L2, as two reductions: the additions happen
+ * there, not in the SM's few FP64 lanes.  (As atomicAdd through a generic
+ * pointer each waited for its answer: 3 us per scatterer.) */
+__device__ __forceinline__ void red_add(double *o, double v) {
+    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(o), "d"(v) : "memory");
+}
+__device__ __forceinline__ void red_add_df(double *o, float h, float l) {
+    red_add(o, wide_of(h));
+    red_add(o, wide_of(l));
+}
+
+/* The compensated sums of an interval [E_j, E_j+1) between two nodes of the
+ * even grid: Sum x and Sum (r - E_j) x of its terms x, per lane, from which
+ * the last block forms every gate exactly (the triangle's end lies where its
+ * table's scale puts it, a few ulps off the node: an interval's own line is
+ * right up to there, where node sums would mix it with its neighbour's).
+ * Doubles acc64[8 j + l] and acc64[8 j + 4 + l]. */
+constexpr unsigned kCompSums = 8;
+
+/* A warp's window of two intervals beside the node E, with t = r - E: below
+ * it (side 0) and above (side 1) the sums of x and of |t| x. */
+struct CompWindow {
+    float Eh, El;
+    int c;              /* the lower interval, -1: none yet */
+    float X[2][4], x[2][4], T[2][4], t[2][4];
+
+    __device__ __forceinline__ void move(const PulseArgs &P, int j) {
+        c = j;
+        comp_node(P, j + 1, Eh, El);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+#pragma unroll
+            for (int l = 0; l < 4; l++) X[q][l] = x[q][l] = T[q][l] = t[q][l] = 0.0f;
+        }
+    }
+    __device__ __forceinline__ void offset(const CompSig &g, float &th, float &tl) const {
+        float e;
+        two_sum(g.r, -Eh, th, e);
+        tl = e + (g.rl - El);
+    }
+    template <int Q>
+    __device__ __forceinline__ void add_side(const CompSig &g, float dh, float dl) {
+#pragma unroll
+        for (int l = 0; l < 4; l++) {
+            float ph, pl;
+            df_acc(X[Q][l], x[Q][l], g.s[l], g.u[l]);
+            df_mul_pair(g.s[l], g.u[l], dh, dl, ph, pl);
+            df_acc(T[Q][l], t[Q][l], ph, pl);
+        }
+    }
+    __device__ __forceinline__ void add(const CompSig &g, float th, float tl) {
+        /* a run in spatial order mostly lies on one side */
+        if (th + tl >= 0.0f) add_side<1>(g, th, tl);
+        else add_side<0>(g, -th, -tl);
+    }
+    __device__ __forceinline__ void flush(const PulseArgs &P, unsigned lane) {
+        if (c < 0) return;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            if (!__any_sync(0xffffffffu, X[q][0] != 0.0f || X[q][1] != 0.0f || X[q][2] != 0.0f || X[q][3] != 0.0f)) continue;
+            float a, b, d, e;
+            warp_sum4_df(lane, X[q], x[q], a, b);
+            warp_sum4_df(lane, T[q], t[q], d, e);
+            if ((lane & 7u) == 0u) {
+                if (q == 0) {
+                    /* |t| = delta - (r - E_j) */
+                    float mh, ml;
+                    df_mul_pair(a, b, P.rdelta, 0.0f, mh, ml);
+                    df_acc(mh, ml, -d, -e);
+                    d = mh;
+                    e = ml;
+                }
+                double *o = P.acc64 + kCompSums * (unsigned)(c + q) + (lane >> 3);
+                red_add_df(o, a, b);
+                red_add_df(o + 4, d, e);
+            }
+        }
+        c = -1;
+    }
+};
+
+/* The interval of a range to one (comp_stray puts it right), -1 off the nodes. */
+__device__ __forceinline__ int comp_interval(const PulseArgs &P, float r) {
+    const int last = (int)node_count(P.G, P.mom_n) - 2;
+    const float jf = floorf((r - P.rs) * P.inv_delta) + (float)P.mom_n;
+    return jf >= -1.0f && jf <= (float)(last + 1) ? min(max((int)jf, 0), last) : -1;
+}
+__device__ __noinline__ void comp_stray(const PulseArgs &P, int j, const CompSig &g) {
+    const float delta = P.rdelta;
+    const int last = (int)node_count(P.G, P.mom_n) - 2;
+    float a, b, c, d, uh, ul;
+    comp_node(P, j, c, d);
+    two_sum(g.r, -c, uh, ul);
+    ul = ul + (g.rl - d);
+    /* the quotient can be one off beside a node */
+    const float u = uh + ul;
+    if (u < 0.0f || u >= delta) {
+        const float by = u < 0.0f ? delta : -delta;
+        j += u < 0.0f ? -1 : 1;
+        two_sum(uh, by, a, b);
+        uh = a;
+        ul = ul + b;
+    }
+    if (j < 0 || j > last || !(uh + ul >= 0.0f && uh + ul <= delta)) return;
+    double *o = P.acc64 + kCompSums * (unsigned)j;
+#pragma unroll 1
+    for (int l = 0; l < 4; l++) {
+        df_mul_pair(g.s[l], g.u[l], uh, ul, a, b);
+        red_add_df(o + l, g.s[l], g.u[l]);
+        red_add_df(o + 4 + l, a, b);
+    }
+}
+
+/* Non-finite values: their lanes of every gate NaN (0 x NaN in pass 1), the
+ * scatterer's finite lanes kept; false when its range is not finite and
+ * nothing is left of it. */
+__device__ __noinline__ bool comp_non_finite(const PulseArgs &P, CompSig &g) {
+    double *gate = P.acc64 + kCompSums * (size_t)node_count(P.G, P.mom_n);
+    const bool range = fabsf(g.r) < INFINITY;
+    for (int l = 0; l < 4; l++) {
+        if (range && fabsf(g.s[l]) < INFINITY && fabsf(g.u[l]) < INFINITY) continue;
+        g.s[l] = g.u[l] = 0.0f;
+        for (unsigned k = 0; k < P.G; k++) atomicAdd(gate + 4 * k + l, (double)NAN);
+    }
+    return range;
+}
+
+/* A run the window does not hold whole: as node_settle. */
+__device__ __forceinline__ void comp_settle(const PulseArgs &P, CompWindow &W, CompSig *g, unsigned in, int part,
+                                            unsigned lane) {
+    int j[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        j[q] = -1;
+        if (!((in >> q) & 1u)) continue;
+        bool live = true;
+        if (!(fabsf(g[q].r) < INFINITY) || !finite4(g[q].s) || !finite4(g[q].u)) live = comp_non_finite(P, g[q]);
+        if (live) j[q] = comp_interval(P, g[q].r);
+    }
+    for (;;) {
+        const unsigned l0 = __ballot_sync(0xffffffffu, j[0] >= 0), l1 = __ballot_sync(0xffffffffu, j[1] >= 0);
+        if ((l0 | l1) == 0u) return;
+        const auto within = [&](int c) {
+            return __popc(__ballot_sync(0xffffffffu, j[0] >= 0 && (unsigned)(j[0] - c) < 2u)) +
+                   __popc(__ballot_sync(0xffffffffu, j[1] >= 0 && (unsigned)(j[1] - c) < 2u));
+        };
+        int here = W.c < 0 ? 0 : within(W.c);
+        if (here < part) {
+            int best = 0, at = 0;
+            unsigned t0 = l0, t1 = l1;
+#pragma unroll 1
+            for (int t = 0; t < 4 && best < part && (t0 | t1) != 0u; t++) {
+                const int src = __ffs(t0 ? t0 : t1) - 1;
+                const int cand = __shfl_sync(0xffffffffu, t0 ? j[0] : j[1], src);
+                const int a = within(cand - 1), b = within(cand);
+                best = max(a, b);
+                at = a > b ? cand - 1 : cand;
+                if (t0) t0 &= ~(0x1ffu << (src & ~7));
+                else t1 &= ~(0x1ffu << (src & ~7));
+            }
+            if (best < part) {
+                if (j[0] >= 0) comp_stray(P, j[0], g[0]);
+                if (j[1] >= 0) comp_stray(P, j[1], g[1]);
+                return;
+            }
+            W.flush(P, lane);
+            W.move(P, min(max(at, 0), (int)node_count(P.G, P.mom_n) - 3));
+        }
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            if (j[q] >= 0 && (unsigned)(j[q] - W.c) < 2u) {
+                float th, tl;
+                W.offset(g[q], th, tl);
+                /* one off beside the window's end: by itself */
+                if (fabsf(th + tl) <= P.rdelta) W.add(g[q], th, tl);
+                else comp_stray(P, j[q], g[q]);
+                j[q] = -1;
+            }
+        }
+    }
+}
 
 /* A scatterer with a non-finite signal reaches every gate, its weight there
  * as pass 1 forms it (0 x NaN is NaN): straight into the grid's sums of the
@@ -250,8 +491,8 @@ __device__ __forceinline__ void node_alone(const PulseArgs &P, const Sig &g, flo
  * and non-finite ones go to every gate; what the window, or one moved to
  * where a good part of the run lies, holds is added to it, and the rest --
  * debris, scatterers respawned elsewhere since the last sort -- one by one. */
-__device__ __forceinline__ void node_settle(const PulseArgs &P, NodeWindow &W, const Sig *g, unsigned in, double *bins,
-                                            float4 *stray, unsigned lane) {
+__device__ __forceinline__ void node_settle(const PulseArgs &P, NodeWindow &W, const Sig *g, unsigned in, int part,
+                                            double *bins, float4 *stray, unsigned lane) {
     int j[2];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
@@ -270,12 +511,12 @@ __device__ __forceinline__ void node_settle(const PulseArgs &P, NodeWindow &W, c
             return __popc(__ballot_sync(0xffffffffu, j[0] >= 0 && (unsigned)(j[0] - c) < 2u)) +
                    __popc(__ballot_sync(0xffffffffu, j[1] >= 0 && (unsigned)(j[1] - c) < 2u));
         };
-        if (W.c < 0 || within(W.c) < kNodePart) {
+        if (W.c < 0 || within(W.c) < part) {
             /* where a few of those left lie: any of them may be astray */
             int best = 0, at = 0;
             unsigned t0 = l0, t1 = l1;
 #pragma unroll 1
-            for (int t = 0; t < 4 && best < kNodePart && (t0 | t1) != 0u; t++) {
+            for (int t = 0; t < 4 && best < part && (t0 | t1) != 0u; t++) {
                 const int src = __ffs(t0 ? t0 : t1) - 1;
                 const int cand = __shfl_sync(0xffffffffu, t0 ? j[0] : j[1], src);
                 const int a = within(cand - 1), b = within(cand);
@@ -285,7 +526,7 @@ __device__ __forceinline__ void node_settle(const PulseArgs &P, NodeWindow &W, c
                 if (t0) t0 &= ~(0x1ffu << (src & ~7));
                 else t1 &= ~(0x1ffu << (src & ~7));
             }
-            if (best < kNodePart) {
+            if (best < part) {
                 if (j[0] >= 0) node_stray(P, stray, j[0], g[0].r, g[0].s);
                 if (j[1] >= 0) node_stray(P, stray, j[1], g[1].r, g[1].s);
                 return;
@@ -305,12 +546,15 @@ __device__ __forceinline__ void node_settle(const PulseArgs &P, NodeWindow &W, c
 
 /* The block's node sums into the grid's accumulator, the last block forming
  * the gates and leaving accumulator and counter at zero. */
+template <int MODE>
 __device__ __forceinline__ void node_finish(const PulseArgs &P, double *bins, unsigned nblk) {
     const unsigned nodes = node_count(P.G, P.mom_n), outs = P.G * 4;
-    __syncthreads();
-    for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) {
-        const double v = bins[o];
-        if (v != 0.0) atomicAdd(P.acc64 + o, v);
+    if (MODE == 0) {
+        __syncthreads();
+        for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) {
+            const double v = bins[o];
+            if (v != 0.0) atomicAdd(P.acc64 + o, v);
+        }
     }
     __shared__ bool s_last;
     __syncthreads();
@@ -322,6 +566,32 @@ __device__ __forceinline__ void node_finish(const PulseArgs &P, double *bins, un
     }
     __syncthreads();
     if (!s_last) return;
+    if constexpr (MODE == 1) {
+        const unsigned all = nodes * kCompSums;
+#pragma unroll 4
+        for (unsigned o = threadIdx.x; o < all; o += blockDim.x) bins[o] = __ldcg(P.acc64 + o);
+        __syncthreads();
+        for (unsigned o = threadIdx.x; o < all; o += blockDim.x) P.acc64[o] = 0.0;
+        const double s = (double)P.rwd[0], ds = (double)P.rdelta * s;
+        for (unsigned o = threadIdx.x; o < outs; o += blockDim.x) {
+            const unsigned k = o >> 2, l = o & 3u, n = (unsigned)P.mom_n;
+            double sum = 0.0;
+            /* gate k lies at index k + n: the intervals n below it, where the
+             * weight is 1 - (m delta - u) s, and n above, 1 - (m delta + u) s */
+            for (unsigned m = 0; m < n; m++) {
+                const double *lo = bins + kCompSums * (k + n - 1 - m) + l, *hi = bins + kCompSums * (k + n + m) + l;
+                sum = fma(1.0 - (double)(m + 1) * ds, lo[0], sum);
+                sum = fma(1.0 - (double)m * ds, hi[0], sum);
+                sum = fma(s, lo[4] - hi[4], sum);
+            }
+            double *extra = P.acc64 + all + o;
+            const double e = __ldcg(extra);
+            if (e != 0.0) *extra = 0.0;
+            reinterpret_cast<float *>(P.pulse)[o] = (float)(sum + e);
+        }
+        if (threadIdx.x == 0) *P.counter = 0u;
+        return;
+    }
     float *sums = reinterpret_cast<float *>(bins), *at_node = sums + 4 * nodes;
     const unsigned copies = node_copies(P.G, P.mom_n);
     const float *stray = reinterpret_cast<const float *>(P.stray);
@@ -361,13 +631,89 @@ __device__ __forceinline__ void node_finish(const PulseArgs &P, double *bins, un
     if (threadIdx.x == 0) *P.counter = 0u;
 }
 
+/* A run of 64 into the warp's window. */
+__device__ __forceinline__ void node_run(const PulseArgs &P, NodeWindow &W, const float4 *p, const float4 *x, unsigned in,
+                                         int part, double *bins, float4 *stray, unsigned lane) {
+    Sig g[2];
+    bool held[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        if (!signal_plain_mid(P, p[q], x[q], g[q])) {
+            Sig32 sg;
+            signal_plain(P, p[q], x[q], sg);
+            g[q].r = sg.r;
+#pragma unroll
+            for (int l = 0; l < 4; l++) g[q].s[l] = sg.s.v[l];
+        }
+        /* NaN or an infinity in any lane makes the sum NaN */
+        const float f = fmaf(g[q].s[0], 0.0f, fmaf(g[q].s[1], 0.0f, fmaf(g[q].s[2], 0.0f, g[q].s[3] * 0.0f)));
+        held[q] = W.holds(g[q].r) && f == 0.0f;
+    }
+    if (__all_sync(0xffffffffu, held[0] && held[1])) {
+        W.add(g[0]);
+        W.add(g[1]);
+    } else if (__popc(__ballot_sync(0xffffffffu, held[0])) + __popc(__ballot_sync(0xffffffffu, held[1])) >=
+               kNodeMost) {
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            if (held[q]) W.add(g[q]);
+            else if ((in >> q) & 1u) node_alone(P, g[q], stray);
+        }
+    } else {
+        node_settle(P, W, g, in, part, bins, stray, lane);
+    }
+}
+__device__ __forceinline__ void comp_run(const PulseArgs &P, CompWindow &W, const float4 *p, const float4 *x, unsigned in,
+                                         int part, unsigned lane) {
+    /* nothing to do when no scatterer of the run reaches a gate and none has
+     * a non-finite value, which would reach all of them */
+    bool live = false;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const float r2 = fmaf(p[q].x, p[q].x, fmaf(p[q].y, p[q].y, p[q].z * p[q].z));
+        const float f = fmaf(x[q].x, 0.0f, fmaf(x[q].y, 0.0f, fmaf(x[q].z, 0.0f, x[q].w * 0.0f)));
+        live = live || !(f == 0.0f && ((r2 > 0x1p-40f && r2 < P.reach_lo2) || (r2 > P.reach_hi2 && r2 < INFINITY)));
+    }
+    if (!__any_sync(0xffffffffu, live)) return;
+    CompSig g[2];
+    float th[2], tl[2];
+    bool held[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        signal_comp_any(P, p[q], x[q], g[q]);
+        /* NaN or an infinity in any lane makes the sum NaN */
+        const float f = fmaf(g[q].s[0], 0.0f, fmaf(g[q].s[1], 0.0f, fmaf(g[q].s[2], 0.0f, g[q].s[3] * 0.0f)));
+        W.offset(g[q], th[q], tl[q]);
+        const float t = th[q] + tl[q];
+        held[q] = t >= -P.rdelta && t < P.rdelta && f == 0.0f;
+    }
+    if (__popc(__ballot_sync(0xffffffffu, held[0])) + __popc(__ballot_sync(0xffffffffu, held[1])) >= kNodeMost) {
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            if (held[q]) {
+                W.add(g[q], th[q], tl[q]);
+            } else if ((in >> q) & 1u) {
+                bool live = true;
+                if (!(fabsf(g[q].r) < INFINITY) || !finite4(g[q].s) || !finite4(g[q].u)) live = comp_non_finite(P, g[q]);
+                const int j = live ? comp_interval(P, g[q].r) : -1;
+                if (j >= 0) comp_stray(P, j, g[q]);
+            }
+        }
+    } else {
+        comp_settle(P, W, g, in, part, lane);
+    }
+}
+
+template <int MODE>   /* RSC_PULSE_PLAIN, RSC_PULSE_COMPENSATED */
 __device__ __forceinline__ void node_body(const PulseArgs &P, unsigned blk, unsigned nblk) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *bins = reinterpret_cast<double *>(smem_raw);
     const unsigned nodes = node_count(P.G, P.mom_n);
     float4 *stray = P.stray + (size_t)nodes * (blk & (node_copies(P.G, P.mom_n) - 1u));
-    for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) bins[o] = 0.0;
-    __syncthreads();
+    if (MODE == 0) {
+        for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) bins[o] = 0.0;
+        __syncthreads();
+    }
     const unsigned lane = threadIdx.x & 31u;
     const unsigned long long n = P.n, runs = (n + 63ull) / 64ull, whole = n / 64ull;
     const unsigned long long warps = (unsigned long long)nblk * (blockDim.x >> 5);
@@ -377,10 +723,17 @@ __device__ __forceinline__ void node_body(const PulseArgs &P, unsigned blk, unsi
     const unsigned long long lead = P.lead / 64ull;
     const unsigned long long last = lead * (me + 1) / warps;
     NodeWindow W;
-    W.c = -1;
-    W.E0 = W.E1 = W.E2 = NAN;
-    W.i0 = W.i1 = 0.0f;
-    W.clear();
+    CompWindow C;
+    if (MODE == 0) {
+        W.c = -1;
+        W.E0 = W.E1 = W.E2 = NAN;
+        W.i0 = W.i1 = 0.0f;
+        W.clear();
+    } else {
+        C.move(P, 0);
+        C.c = -1;
+        C.Eh = NAN;
+    }
     const auto next = [&](unsigned long long r) {
         r++;
         return r == last ? lead + me : (r > last ? r + (warps - 1) : r);
@@ -407,41 +760,24 @@ __device__ __forceinline__ void node_body(const PulseArgs &P, unsigned blk, unsi
                 if (past) in &= ~(1u << q);
             }
         }
-        Sig g[2];
-        bool held[2];
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            if (!signal_plain_mid(P, p[q], x[q], g[q])) {
-                Sig32 sg;
-                signal_plain(P, p[q], x[q], sg);
-                g[q].r = sg.r;
-#pragma unroll
-                for (int l = 0; l < 4; l++) g[q].s[l] = sg.s.v[l];
-            }
-            /* NaN or an infinity in any lane makes the sum NaN */
-            const float f = fmaf(g[q].s[0], 0.0f, fmaf(g[q].s[1], 0.0f, fmaf(g[q].s[2], 0.0f, g[q].s[3] * 0.0f)));
-            held[q] = W.holds(g[q].r) && f == 0.0f;
-        }
-        if (__all_sync(0xffffffffu, held[0] && held[1])) {
-            W.add(g[0]);
-            W.add(g[1]);
-        } else if (__popc(__ballot_sync(0xffffffffu, held[0])) + __popc(__ballot_sync(0xffffffffu, held[1])) >=
-                   kNodeMost) {
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                if (held[q]) W.add(g[q]);
-                else if ((in >> q) & 1u) node_alone(P, g[q], stray);
-            }
+        const int part = run < lead ? kNodePart : kNodeMost;
+        if constexpr (MODE == 0) {
+            node_run(P, W, p, x, in, part, bins, stray, lane);
         } else {
-            node_settle(P, W, g, in, bins, stray, lane);
+            comp_run(P, C, p, x, in, part, lane);
         }
     }
-    W.flush(bins, lane);
-    node_finish(P, bins, nblk);
+    if (MODE == 0) W.flush(bins, lane);
+    else C.flush(P, lane);
+    node_finish<MODE>(P, bins, nblk);
 }
 
 __global__ void __launch_bounds__(kNodeThreads, kNodeMinBlocks) k_pulse_nodes(const PulseArgs P) {
-    node_body(P, blockIdx.x, gridDim.x);
+    node_body<0>(P, blockIdx.x, gridDim.x);
+}
+
+__global__ void __launch_bounds__(kNodeThreads, kCompMinBlocks) k_pulse_nodes_comp(const PulseArgs P) {
+    node_body<1>(P, blockIdx.x, gridDim.x);
 }
 
 }  // namespace rsc

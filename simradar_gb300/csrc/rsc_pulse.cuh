@@ -451,6 +451,209 @@ __device__ __forceinline__ void signal_comp(const PulseArgs &P, float4 p, float4
     o.r_lo = rl;
 }
 
+/* A scatterer's compensated signal: range and terms as double-floats. */
+struct CompSig {
+    float r, rl, s[4], u[4];
+};
+
+/* sine and cosine of rh + rl + q pi/2 (|rh| <= 0.8, |rl| <= ulp(rh)) as
+ * double-floats, by their Taylor series: the terms r, r^3/6, r^5/120,
+ * 1 - r^2/2 and r^4/24 as double-floats, the rest (below 4e-4) in FP32, rl to
+ * first order.  Within 1e-10, rms 1e-11: the range's own 2^-48 leaves the
+ * phase 3e-10 rad (rms) at 2 km and 5e-9 at 30 km, which the 1e-14 of
+ * sincos_df's node table, at twice the operations, cannot better.  qbits: q
+ * in its low bits. */
+__device__ __forceinline__ void sincos_series_df(float rh, float rl, unsigned qbits, float &sh, float &sl, float &ch,
+                                                 float &cl) {
+    float p, pe;
+    two_prod(rh, rh, p, pe);
+    /* -r^3 / 6 and the rest of the sine */
+    const float t = p * rh, tl = fmaf(pe, rh, fmaf(p, rh, -t));
+    const float c3 = t * -0x1.555556p-3f;
+    const float c3l = fmaf(t, -0x1.555556p-3f, -c3) + fmaf(t, 0x1.555556p-28f, tl * -0x1.555556p-3f);
+    const float t5 = t * p, t5l = fmaf(tl, p, fmaf(t, p, -t5));   /* r^5 */
+    const float c5 = t5 * 0x1.111112p-7f;
+    const float c5l = fmaf(t5, 0x1.111112p-7f, -c5) + fmaf(t5, -0x1.dddddep-32f, t5l * 0x1.111112p-7f);
+    float ps = fmaf(p, -0x1.ae6456p-26f, 0x1.71de3ap-19f);
+    ps = fmaf(ps, p, -0x1.a01a02p-13f);
+    /* 1 - r^2 / 2, r^4 / 24 and the rest of the cosine */
+    const float h = -0.5f * p, p2 = p * p;
+    const float c4 = p2 * 0x1.555556p-5f;
+    const float c4l = fmaf(p2, 0x1.555556p-5f, -c4) +
+                      fmaf(p2, -0x1.555556p-30f, (fmaf(p, p, -p2) + 2.0f * p * pe) * 0x1.555556p-5f);
+    float pc = fmaf(p, 0x1.1eed8ep-29f, -0x1.27e4fcp-22f);
+    pc = fmaf(pc, p, 0x1.a01a02p-16f);
+    pc = fmaf(pc, p, -0x1.6c16c2p-10f);
+    float s0, se, s2, s2e, c0, ce, c1, c1e;
+    fast_two_sum(rh, c3, s2, s2e);
+    fast_two_sum(s2, c5, s0, se);
+    fast_two_sum(1.0f, h, c0, ce);
+    fast_two_sum(c0, c4, c1, c1e);
+    const float s1 = (se + s2e) + (fmaf(t5 * p, ps, c3l + c5l) + rl * c1);
+    const float c2 = (ce + c1e) + (fmaf(p2 * p, pc, c4l) - fmaf(0.5f, pe, rl * s0));
+    const bool swap = (qbits & 1u) != 0u;
+    const unsigned fs = (qbits & 2u) << 30, fc = ((qbits + 1u) & 2u) << 30;
+    sh = __uint_as_float(__float_as_uint(swap ? c1 : s0) ^ fs);
+    sl = __uint_as_float(__float_as_uint(swap ? c2 : s1) ^ fs);
+    ch = __uint_as_float(__float_as_uint(swap ? s0 : c1) ^ fc);
+    cl = __uint_as_float(__float_as_uint(swap ? s1 : c2) ^ fc);
+}
+
+/* signal_comp for scatterers ahead of the beam whose antenna weight lies
+ * within 16 degrees of it, or past the table's end: the same quantities as
+ * double-floats by fewer operations.
+ *   range      sqrt of the exact squares, its tail from the residual
+ *   angle      theta^2 = asin^2(sqrt S) = S (1 + S/3 + 8 S^2/45 + ...) of
+ *              S = |b x p|^2 / (|b|^2 r^2): no quotient and one root, where
+ *              asin of the sine takes two roots, a quotient and its own series
+ *   phase      reduced as in reduce_pio2_df, sine and cosine by series
+ * False (o not formed) elsewhere: the caller takes signal_comp. */
+__device__ __forceinline__ bool signal_comp_mid(const PulseArgs &P, const float4 &p, const float4 &x, CompSig &o) {
+    const float *sd = P.sim;
+    float a, ae, b, be, c, ce, h, e, h2, e2;
+    two_prod(p.x, p.x, a, ae);
+    two_prod(p.y, p.y, b, be);
+    two_prod(p.z, p.z, c, ce);
+    two_sum(a, b, h, e);
+    two_sum(h, c, h2, e2);
+    float r2h, r2l;
+    fast_two_sum(h2, (e + e2) + (ae + be + ce), r2h, r2l);
+    const float yr = rsqrt_approx(r2h), rh = sqrt_from(r2h, yr);
+    const float rn = fmaf(-rh, rh, r2h) + r2l, hy = 0.5f * yr, ra = rn * hy;
+    const float rl = fmaf(fmaf(-rh, 2.0f * ra, rn), hy, ra);
+    const float ath = rcp_mid(r2h), atl = ath * fmaf(-r2l, ath, fmaf(-r2h, ath, 1.0f));   /* 1 / r^2 */
+    /* S */
+    const float bx = sd[0], by = sd[1], bz = sd[2];
+    float Sh, Sl;
+    {
+        float vh[3], vl[3];
+        const float m[3][4] = {{by, p.z, bz, p.y}, {bz, p.x, bx, p.z}, {bx, p.y, by, p.x}};
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            float p1, e1, q1, f1, d;
+            two_prod(m[k][0], m[k][1], p1, e1);
+            two_prod(m[k][2], m[k][3], q1, f1);
+            two_sum(p1, -q1, vh[k], d);
+            vl[k] = d + (e1 - f1);
+            two_prod(vh[k], vh[k], p1, e1);
+            vl[k] = fmaf(2.0f * vh[k], vl[k], e1);
+            vh[k] = p1;
+        }
+        float s1, f1, s2, f2;
+        two_sum(vh[0], vh[1], s1, f1);
+        two_sum(s1, vh[2], s2, f2);
+        float kh, kl;
+        df_mul_pair(ath, atl, P.ib2_hi, P.ib2_lo, kh, kl);
+        df_mul_pair(s2, (f1 + f2) + (vl[0] + vl[1] + vl[2]), kh, kl, Sh, Sl);
+    }
+    float q = fmaf(Sh, 0x1.d0ef1ap-6f, 0x1.10a580p-5f);   /* 2^(2n-1) / (n^2 C(2n, n)), n = 10, 9, .. 4 */
+    q = fmaf(q, Sh, 0x1.45e5d2p-5f);
+    q = fmaf(q, Sh, 0x1.8f0ef8p-5f);
+    q = fmaf(q, Sh, 0x1.f85d96p-5f);
+    q = fmaf(q, Sh, 0x1.4ce19ap-4f);
+    q = fmaf(q, Sh, 0x1.d41d42p-4f);
+    const float t3 = Sh * 0x1.555556p-2f;   /* S / 3 and 8 S^2 / 45 as double-floats */
+    const float t3l = fmaf(Sh, 0x1.555556p-2f, -t3) + fmaf(Sh, -0x1.555556p-27f, Sl * 0x1.555556p-2f);
+    const float S2 = Sh * Sh, S2l = fmaf(2.0f * Sh, Sl, fmaf(Sh, Sh, -S2));
+    const float t5 = S2 * 0x1.6c16c2p-3f;
+    const float t5l = fmaf(S2, 0x1.6c16c2p-3f, -t5) + fmaf(S2, -0x1.27d27ep-28f, S2l * 0x1.6c16c2p-3f);
+    float th, tl, oh, ol, th2, tl2;
+    fast_two_sum(t3, t5, th, tl);
+    tl = tl + fmaf(S2 * Sh, q, t5l);
+    fast_two_sum(1.0f, th, oh, ol);
+    df_mul_pair(Sh, Sl, oh, ol + (tl + t3l), th, tl);
+    fast_two_sum(th, tl, th2, tl2);   /* the root below takes its tail to first order */
+    const float yt = rsqrt_approx(fmaxf(th2, 0x1p-100f));
+    const float gh = th2 * yt, gl = (fmaf(-gh, gh, th2) + tl2) * (0.5f * yt);   /* theta */
+    /* the antenna weight (weight_comp_df); past the end the series falls
+     * short of the angle, never past it */
+    const float dot = fmaf(bx, p.x, fmaf(by, p.y, bz * p.z));
+    const float ws = P.awd[0], wo = P.awd[1], wm = P.awd[2];
+    const float f0 = gh * ws;
+    float f, fe;
+    two_sum(f0, wo, f, fe);
+    fe = fe + fmaf(gl, ws, fmaf(gh, ws, -f0));
+    const float fsum = f + fe;
+    const float phase = sd[4] * rh;
+    const bool mid = dot > 0.0f && ws > 0.0f && (Sh < 0.08f || fsum >= wm + 1.0f) && r2h > 0x1p-60f &&
+                     r2h < 0x1p60f && fabsf(phase) < 0x1p22f;
+    float wah, wal;
+    {
+        const float fc = fminf(fmaxf(fsum, 0.0f), wm), fl = floorf(fc);
+        const int i0 = (int)fl;
+        const float w0 = __ldg(P.aw + i0), w1 = __ldg(P.aw + min(i0 + 1, (int)wm));
+        const bool edge = !(fsum > 0.0f && fsum < wm);
+        float dh, dl, ph, pl;
+        two_sum(w1, -w0, dh, dl);
+        df_mul_pair(dh, dl, edge ? 0.0f : f - fl, edge ? 0.0f : fe, ph, pl);
+        float we;
+        two_sum(w0, ph, wah, we);
+        wal = we + pl;
+    }
+    float kh, kl;
+    df_mul_pair(ath, atl, wah, wal, kh, kl);
+    /* the phase k rh + k rl less q pi/2 (reduce_pio2_df) */
+    float xl, pa, pb, xsh, xse;
+    xl = fmaf(sd[4], rh, -phase);
+    two_prod(sd[4], rl, pa, pb);
+    two_sum(xl, pa, xsh, xse);
+    const float magic = 12582912.0f;   /* 1.5 x 2^23 */
+    const float qp = phase * RSM_TWO_OVER_PI;
+    const float q0 = __fadd_rn(qp, magic) - magic;
+    const float fr = (qp - q0) + fmaf(xsh, RSM_TWO_OVER_PI, fmaf(phase, 0x1.b93910p-26f, fmaf(phase, RSM_TWO_OVER_PI, -qp)));
+    const float qq = q0 + (__fadd_rn(fr, magic) - magic);
+    const unsigned qbits = __float_as_uint(__fadd_rn(qq, magic));
+    const float r1 = fmaf(-qq, RSM_PIO2_1, phase);
+    float u, ue, v, ve, w, we;
+    two_prod(qq, RSM_PIO2_2, u, ue);
+    two_sum(r1, -u, v, ve);
+    two_sum(v, xsh, w, we);
+    float redh, redl;
+    fast_two_sum(w, we + ((ve - ue) + fmaf(-qq, RSM_PIO2_3, xse + pb)), redh, redl);
+    float ssh, ssl, cch, ccl;
+    sincos_series_df(redh, redl, qbits, ssh, ssl, cch, ccl);
+    /* attenuation x antenna weight joins the sine and cosine, then the rotation */
+    float ckh, ckl, skh, skl;
+    df_mul_pair(cch, ccl, kh, kl, ckh, ckl);
+    df_mul_pair(ssh, ssl, kh, kl, skh, skl);
+    const float xa[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int l = 0; l < 4; l++) {
+        const float s0 = xa[l], s1 = (l & 1) ? -xa[l - 1] : xa[l + 1];
+        float p1, e1, p2, f1, d;
+        two_prod(s0, ckh, p1, e1);
+        two_prod(s1, skh, p2, f1);
+        two_sum(p1, p2, o.s[l], d);
+        o.u[l] = d + fmaf(s0, ckl, fmaf(s1, skl, e1 + f1));
+    }
+    o.r = rh;
+    o.rl = rl;
+    return mid;
+}
+
+/* The compensated signal: signal_comp_mid where it holds, else signal_comp. */
+__device__ __forceinline__ void signal_comp_any(const PulseArgs &P, const float4 &p, const float4 &x, CompSig &o) {
+    if (signal_comp_mid(P, p, x, o)) return;
+    Sig32 sg;
+    signal_comp(P, p, x, sg);
+    o.r = sg.r;
+    o.rl = sg.r_lo;
+#pragma unroll
+    for (int l = 0; l < 4; l++) {
+        o.s[l] = sg.s.v[l];
+        o.u[l] = sg.s_lo[l];
+    }
+}
+__device__ __forceinline__ void signal_comp_any(const PulseArgs &P, float4 p, float4 x, Sig32 &o) {
+    CompSig g;
+    signal_comp_any(P, p, x, g);
+    o.r = g.r;
+    o.r_lo = g.rl;
+    o.s.set(g.s[0], g.s[1], g.s[2], g.s[3]);
+#pragma unroll
+    for (int l = 0; l < 4; l++) o.s_lo[l] = g.u[l];
+}
+
 template <int MODE>  /* RSC_PULSE_PLAIN, RSC_PULSE_COMPENSATED, RSC_PULSE_F64 */
 struct PulseTraits;
 template <> struct PulseTraits<0> { typedef AccF32 Acc; static constexpr unsigned kMain = kBinStride32; };
@@ -648,7 +851,7 @@ struct PulseBins {
                 if constexpr (MODE == 0) {
                     signal_plain(P, p, x, sg);
                 } else {
-                    signal_comp(P, p, x, sg);
+                    signal_comp_any(P, p, x, sg);
                 }
                 c.set(sg.s.v[0], sg.s.v[1], sg.s.v[2], sg.s.v[3]);
                 if constexpr (MODE == 1) c.set_lo(sg.s_lo);
@@ -924,7 +1127,7 @@ struct PulseBins {
                 if constexpr (MODE == 0) {
                     signal_plain(P, pp[q], xx[q], sg);
                 } else {
-                    signal_comp(P, pp[q], xx[q], sg);
+                    signal_comp_any(P, pp[q], xx[q], sg);
                 }
                 const bool fin = fabsf(sg.r) < INFINITY && finite4(sg.s.v);
                 bad = bad || !fin;

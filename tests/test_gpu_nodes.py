@@ -102,3 +102,31 @@ def test_mid_range_roots_and_quotients(backend):
     assert np.array_equal(backend.eval_math(13, a), np.sqrt(a))
     assert np.array_equal(backend.eval_math(14, a, b), a / b)
     assert np.array_equal(backend.eval_math(14, np.ones_like(b), b), np.float32(1.0) / b)
+
+
+@pytest.mark.parametrize("spacing,gates,rain,debris", [
+    (30.0, 20, 256, 0), (7.5, 77, 4097, 3000), (2.5, 240, 9001, 0), (1.5, 512, 1999, 33), (15.0, 1, 777, 0),
+])
+def test_compensated_node_sums(backend, oracle_lib, spacing, gates, rain, debris):
+    """The compensated pulse of every half width of the triangle against FP64:
+    5e-9 of the sum of |w x| for the terms (the range to 2e-14 in the phase of
+    2.5e5 rad; the sine and cosine add 1e-10), and the output's own
+    rounding of its component."""
+    O = oracle_lib
+    objs = [(synth.OBJ_LEAF, debris), (synth.OBJ_BRICK, debris // 2 + 1)] if debris else []
+    S = synth.make_scene(num_rain=rain, debris=objs, gates=gates, gate_spacing=spacing, les_count=1, seed=5)
+    pop = synth.population(S)
+    W = backend.Worker(0)
+    synth.load_worker(W, S)
+    W.set_precision(1)
+    st = O.OracleState(S.state)
+    for k in range(3):
+        sd = synth.pulse_sim_desc(S, 40 + k)
+        W.make_pulse(sd)
+        g = W.download_pulse(1.0).astype(np.float64)
+        r64, ab = O.make_pulse_f64(st, S, sd, return_abs=True)
+        lim = 5.0e-9 * ab + 6.0e-8 * np.abs(r64) + 1e-30
+        assert (np.abs(g - r64) <= lim).all(), "pulse %d: worst %g of the bound" % (k, (np.abs(g - r64) / lim).max())
+        W.advance_time(pop, 0, sd)
+        O.advance_time(st, S, S.counts, S.les[0], sd)
+    W.close()
