@@ -22,6 +22,7 @@
 #include "rsc_sort.cuh"
 #include "rsc_les.h"
 #include "rsc_populate.h"
+#include "rsc_popgen.cuh"
 
 using rsc::AdvanceArgs;
 using rsc::DebrisType;
@@ -1381,6 +1382,12 @@ __global__ void __launch_bounds__(256) k_fill_population(float4 *vel, float4 *or
 
 extern "C" {
 
+/* Scatterers per chunk of draws: `least`, or more so that the host forms at
+ * most 4096 chunks' states. */
+static unsigned pop_per_chunk(size_t n, size_t least) {
+    return (unsigned)std::max<size_t>(least, ((n + 4095) / 4096 + 31) / 32 * 32);
+}
+
 int rsc_populate_upload(rsc_worker *w, const rsc_populate_args *args, uint32_t *dsd_pop) {
     int s = check_alloc(w);
     if (s) return s;
@@ -1395,29 +1402,62 @@ int rsc_populate_upload(rsc_worker *w, const rsc_populate_args *args, uint32_t *
     if (dsd_pop && args->dsd_count) memset(dsd_pop, 0, args->dsd_count * sizeof(uint32_t));
     RSC_CUDA(cudaStreamSynchronize(w->stream));
     free_sort(w);   /* the state is replaced: slots in the caller's order again */
-    const size_t chunk = (size_t)1 << 20;
-    float *hp[2] = {nullptr, nullptr}, *ha[2] = {nullptr, nullptr};
-    uint32_t *hr[2] = {nullptr, nullptr};
-    cudaEvent_t ev[2] = {nullptr, nullptr};
-    cudaError_t e = cudaSuccess;
-    for (int b = 0; b < 2 && e == cudaSuccess; b++) {
-        e = cudaMallocHost((void **)&hp[b], chunk * 16);
-        if (e == cudaSuccess) e = cudaMallocHost((void **)&ha[b], chunk * 16);
-        if (e == cudaSuccess) e = cudaMallocHost((void **)&hr[b], chunk * 16);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev[b], cudaEventDisableTiming);
+    /* the words at the start of every chunk of draws, the drop sizes and
+     * their counts, in one device buffer for this call */
+    const size_t rain = args->dsd_count > 0 ? (size_t)args->counts[0] : 0;
+    const unsigned per_s = pop_per_chunk(g.total, 1024), per_r = pop_per_chunk(rain, 4096);
+    const unsigned chunks_s = (unsigned)((g.total + per_s - 1) / per_s), chunks_r = (unsigned)((rain + per_r - 1) / per_r);
+    std::vector<uint32_t> host((size_t)(chunks_s + chunks_r) * rsc::kPopWords + 3 * (size_t)args->dsd_count);
+    rscpop::chunk_states(&g.main_rs, 8ull * per_s, chunks_s, host.data());
+    uint32_t *h_r = host.data() + (size_t)chunks_s * rsc::kPopWords, *h_dsd = h_r + (size_t)chunks_r * rsc::kPopWords;
+    rscpop::chunk_states(&g.dsd_rs, per_r, chunks_r, h_r);
+    if (args->dsd_count) {
+        memcpy(h_dsd, args->dsd_r, args->dsd_count * sizeof(float));
+        memcpy(h_dsd + args->dsd_count, args->dsd_cdf, args->dsd_count * sizeof(float));
+        memset(h_dsd + 2 * (size_t)args->dsd_count, 0, args->dsd_count * sizeof(uint32_t));
     }
-    bool used[2] = {false, false};
-    for (size_t c = 0; e == cudaSuccess && c < g.total; c += chunk) {
-        const int b = (int)((c / chunk) & 1);
-        if (used[b]) e = cudaEventSynchronize(ev[b]);   /* the copies out of this buffer are done */
-        if (e != cudaSuccess) break;
-        const size_t n = g.total - c < chunk ? g.total - c : chunk;
-        g.fill(n, hp[b], ha[b], hr[b], dsd_pop);   /* overlaps the copies of the other buffer */
-        e = cudaMemcpyAsync(w->pos + c, hp[b], n * 16, cudaMemcpyHostToDevice, w->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(w->aux + c, ha[b], n * 16, cudaMemcpyHostToDevice, w->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(w->rnd + c, hr[b], n * 16, cudaMemcpyHostToDevice, w->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(ev[b], w->stream);
-        used[b] = true;
+    uint32_t *dev = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (!host.empty()) {
+        e = cudaMalloc((void **)&dev, host.size() * sizeof(uint32_t));
+        if (e != cudaSuccess) return cuda_fail(RSC_ERR_NOMEM, "populate: %zu B: %s", host.size() * 4, cudaGetErrorString(e));
+        e = cudaMemcpyAsync(dev, host.data(), host.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, w->stream);
+    }
+    rsc::PopArgs a;
+    memset(&a, 0, sizeof(a));
+    a.pos = w->pos;
+    a.aux = w->aux;
+    a.rnd = w->rnd;
+    for (int k = 0; k < 3; k++) {
+        a.origin[k] = args->domain_origin[k];
+        a.size[k] = args->domain_size[k];
+    }
+    if (e == cudaSuccess && chunks_s) {
+        a.states = dev;
+        a.total = g.total;
+        a.per_chunk = per_s;
+        a.chunks = chunks_s;
+        rsc::k_pop_scatterers<<<grid_of(chunks_s, rsc::kPopWarps), 32 * rsc::kPopWarps, 0, w->stream>>>(a);
+        e = cudaGetLastError();
+        w->launches++;
+    }
+    uint32_t *d_dsd = dev + (h_dsd - host.data());
+    if (e == cudaSuccess && chunks_r) {
+        a.states = dev + (h_r - host.data());
+        a.total = rain;
+        a.per_chunk = per_r;
+        a.chunks = chunks_r;
+        a.dsd_r = reinterpret_cast<const float *>(d_dsd);
+        a.dsd_cdf = a.dsd_r + args->dsd_count;
+        a.dsd_count = args->dsd_count;
+        a.uniform = (args->sim_concept & rsc::kConceptUniformDSD) ? 1 : 0;
+        a.pop = d_dsd + 2 * (size_t)args->dsd_count;
+        rsc::k_pop_sizes<<<grid_of(chunks_r, rsc::kPopWarps), 32 * rsc::kPopWarps, 0, w->stream>>>(a);
+        e = cudaGetLastError();
+        w->launches++;
+        if (e == cudaSuccess && dsd_pop) {
+            e = cudaMemcpyAsync(dsd_pop, a.pop, args->dsd_count * sizeof(uint32_t), cudaMemcpyDeviceToHost, w->stream);
+        }
     }
     const size_t tail = w->numel - g.total;
     if (e == cudaSuccess && tail) e = cudaMemsetAsync(w->pos + g.total, 0, tail * 16, w->stream);
@@ -1430,12 +1470,7 @@ int rsc_populate_upload(rsc_worker *w, const rsc_populate_args *args, uint32_t *
         w->launches++;
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(w->stream);
-    for (int b = 0; b < 2; b++) {
-        if (hp[b]) cudaFreeHost(hp[b]);
-        if (ha[b]) cudaFreeHost(ha[b]);
-        if (hr[b]) cudaFreeHost(hr[b]);
-        if (ev[b]) cudaEventDestroy(ev[b]);
-    }
+    free_ptr(dev);
     if (e != cudaSuccess) return cuda_fail(RSC_ERR_CUDA, "populate: %s", cudaGetErrorString(e));
     w->sig_aux_stale = false;
     w->have_pulse_desc = false;

@@ -58,6 +58,45 @@ int32_t rand_next(RandState *s) {
     return (int32_t)(v >> 1);
 }
 
+namespace {
+constexpr int kOrder = 31;   /* r[i] = r[i - 3] + r[i - 31]: x^31 = x^28 + 1 */
+
+/* c = a b mod (x^31 - x^28 - 1), coefficients mod 2^32 */
+void mul_mod(const uint32_t *a, const uint32_t *b, uint32_t *c) {
+    uint32_t t[2 * kOrder - 1] = {0};
+    for (int i = 0; i < kOrder; i++) {
+        for (int j = 0; j < kOrder; j++) t[i + j] += a[i] * b[j];
+    }
+    for (int i = 2 * kOrder - 2; i >= kOrder; i--) {
+        t[i - 3] += t[i];
+        t[i - kOrder] += t[i];
+    }
+    memcpy(c, t, kOrder * sizeof(uint32_t));
+}
+}  // namespace
+
+void chunk_states(const RandState *s, uint64_t per, size_t chunks, uint32_t *out) {
+    if (chunks == 0) return;
+    /* the last 31 words generated, oldest first */
+    for (int k = 0; k < kOrder; k++) out[k] = s->r[(s->pos + 34 - kOrder + k) % 34];
+    /* x^per by squaring */
+    uint32_t jump[kOrder] = {1}, sq[kOrder] = {0, 1};
+    for (uint64_t e = per; e != 0; e >>= 1) {
+        if (e & 1u) mul_mod(jump, sq, jump);
+        mul_mod(sq, sq, sq);
+    }
+    for (size_t c = 1; c < chunks; c++) {
+        const uint32_t *last = out + (c - 1) * kOrder;
+        uint32_t w[2 * kOrder - 1], next[kOrder] = {0};
+        memcpy(w, last, kOrder * sizeof(uint32_t));
+        for (int i = kOrder; i < 2 * kOrder - 1; i++) w[i] = w[i - 3] + w[i - kOrder];
+        for (int k = 0; k < kOrder; k++) {
+            for (int j = 0; j < kOrder; j++) next[j] += jump[k] * w[k + j];
+        }
+        memcpy(out + c * kOrder, next, sizeof(next));
+    }
+}
+
 int Generator::init(const rsc_populate_args *args, const char **why) {
     a = *args;
     if (a.num_types < 1 || a.num_types > RSC_MAX_TYPES) {
@@ -101,6 +140,7 @@ void Generator::fill(size_t n, float *pos4, float *aux4, uint32_t *rnd4, uint32_
             int bin = 0;
             if (a.sim_concept & 0x10u) {   /* uniform DSD, scaled RCS */
                 bin = (int)(u * (float)a.dsd_count);
+                if (bin >= (int)a.dsd_count) bin = (int)a.dsd_count - 1;   /* u rounds to 1 */
             } else {
                 for (int k = (int)a.dsd_count - 1; k >= 0; k--) {
                     if (u >= a.dsd_cdf[k]) {

@@ -21,6 +21,11 @@ struct RandState {
 void rand_seed(RandState *s, uint32_t seed);
 int32_t rand_next(RandState *s);
 
+/* The 31 words before draw c * per of the sequence, for c = 0 .. chunks - 1
+ * (out: chunks x 31), each from the last by the coefficients of x^per mod
+ * (x^31 - x^28 - 1). */
+void chunk_states(const RandState *s, uint64_t per, size_t chunks, uint32_t *out);
+
 /* RS_populate's draws in slot order for one worker whose type ranges follow
  * one another from slot 0 (origins[k] = counts[0] + ... + counts[k-1]). */
 struct Generator {
