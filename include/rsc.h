@@ -162,8 +162,8 @@ int rsc_synchronize(rsc_worker *w);
 
 /* The latest pulse copied to pulse4 (range_count float4, no gain) without
  * waiting: the copy runs on a stream of its own once the pulse is formed, so
- * the next advance does not wait for it (the next pulse does), and it is
- * complete after rsc_synchronize.  With page-locked pulse4 the host can queue
+ * the next steps do not wait for it (the fourth pulse after it does), and it
+ * is complete after rsc_synchronize.  With page-locked pulse4 the host can queue
  * the next pulses while earlier copies are in flight (additive; the
  * reference reads each pulse with a blocking clEnqueueReadBuffer, rs.c:5115). */
 int rsc_download_pulse_async(rsc_worker *w, float *pulse4);

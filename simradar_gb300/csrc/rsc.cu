@@ -71,6 +71,12 @@ struct Table2D {
 
 }  // namespace
 
+/* Pulses a worker keeps, so that one on its way to the host does not hold up
+ * the next: the copy's latency stood between every two pulses of a loop that
+ * queues them (12 steps of 131,072 scatterers: 456 us over one buffer, 379
+ * over four; 2M, where the advance sets the pace: no difference). */
+constexpr int kPulseRing = 4;
+
 struct rsc_worker {
     int device = 0;
     int num_sms = 0;
@@ -170,11 +176,14 @@ struct rsc_worker {
     int geo_grid = 0, geo_threads = 0;
     size_t geo_smem = 0;
     /* rsc_download_pulse_async: the pulse goes to the host on its own stream,
-     * so the next advance does not wait for the copy; the next pulse kernel
-     * (which rewrites the pulse) waits for d2h_done */
+     * so neither the next advance nor the next pulse waits for the copy: a
+     * pulse that would overwrite one under way goes to the next of a ring */
     cudaStream_t d2h = nullptr;
-    cudaEvent_t pulse_ev = nullptr, d2h_done = nullptr;
-    bool d2h_pending = false;
+    cudaEvent_t pulse_ev = nullptr;
+    float4 *pulse_ring = nullptr;         /* kPulseRing pulses; `pulse` is the latest's, at pulse_at */
+    int pulse_at = 0;
+    cudaEvent_t d2h_done[kPulseRing] = {nullptr};
+    bool d2h_busy[kPulseRing] = {false};  /* a copy of that pulse may be under way */
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     bool pend = false;
     AdvanceArgs pend_a;
@@ -264,7 +273,7 @@ void attribute_arrays(rsc_worker *w, uint4 **out[8]) {
 void free_arrays(rsc_worker *w) {
     if (w->d2h) cudaStreamSynchronize(w->d2h);
     if (w->adv) cudaStreamSynchronize(w->adv);
-    w->d2h_pending = false;
+    for (bool &b : w->d2h_busy) b = false;
     w->read_pending = w->read_next_pending = w->main_pending = false;
     free_ptr(w->pos_next);
     free_ptr(w->rcs_next);
@@ -277,7 +286,9 @@ void free_arrays(rsc_worker *w) {
     free_ptr(w->rcs);
     free_ptr(w->sig);
     free_ptr(w->rnd);
-    free_ptr(w->pulse);
+    free_ptr(w->pulse_ring);
+    w->pulse_ring = nullptr;
+    w->pulse_at = 0;
     free_ptr(w->pulse64);
     free_ptr(w->rk);
     free_ptr(w->rk_hi);
@@ -833,7 +844,9 @@ int rsc_worker_free(rsc_worker *w) {
         cudaStreamDestroy(w->d2h);
     }
     if (w->pulse_ev) cudaEventDestroy(w->pulse_ev);
-    if (w->d2h_done) cudaEventDestroy(w->d2h_done);
+    for (cudaEvent_t e : w->d2h_done) {
+        if (e) cudaEventDestroy(e);
+    }
     if (w->adv) cudaStreamDestroy(w->adv);
     cudaEvent_t evs[] = {w->ev_read, w->ev_read_next, w->ev_adv, w->ev_main};
     for (cudaEvent_t e : evs) {
@@ -878,8 +891,9 @@ int rsc_worker_malloc(rsc_worker *w, size_t num_scats, float range_start, float 
     }
     RSC_CUDA(cudaMalloc((void **)&w->rnd, numel * sizeof(uint4)));
     RSC_CUDA(cudaMemsetAsync(w->rnd, 0, numel * sizeof(uint4), w->stream));
-    RSC_CUDA(cudaMalloc((void **)&w->pulse, range_count * sizeof(float4)));
-    RSC_CUDA(cudaMemsetAsync(w->pulse, 0, range_count * sizeof(float4), w->stream));
+    RSC_CUDA(cudaMalloc((void **)&w->pulse_ring, kPulseRing * range_count * sizeof(float4)));
+    RSC_CUDA(cudaMemsetAsync(w->pulse_ring, 0, kPulseRing * range_count * sizeof(float4), w->stream));
+    w->pulse = w->pulse_ring;
     RSC_CUDA(cudaMalloc((void **)&w->pulse64, range_count * 4 * sizeof(double)));
     RSC_CUDA(cudaMalloc((void **)&w->rk, range_count * sizeof(float)));
     RSC_CUDA(cudaMalloc((void **)&w->rk_hi, range_count * sizeof(float)));
@@ -954,13 +968,18 @@ int rsc_set_rcs_ellipsoid(rsc_worker *w, const float *table4, uint32_t n, const 
     return release_main(w);
 }
 
-/* The worker's stream waits for an asynchronous pulse copy before the pulse
- * is rewritten. */
-static int pulse_d2h_wait(rsc_worker *w) {
-    if (!w->d2h_pending) return RSC_OK;
-    RSC_CUDA(cudaStreamWaitEvent(w->stream, w->d2h_done, 0));
-    w->d2h_pending = false;
+/* Where the next pulse goes: over the latest one unless a copy of that may be
+ * under way, else into the next of the ring, once its own copy is done. */
+static int pulse_slot(rsc_worker *w, int *slot) {
+    *slot = w->d2h_busy[w->pulse_at] ? (w->pulse_at + 1) % kPulseRing : w->pulse_at;
+    if (!w->d2h_busy[*slot]) return RSC_OK;
+    RSC_CUDA(cudaStreamWaitEvent(w->stream, w->d2h_done[*slot], 0));
+    w->d2h_busy[*slot] = false;
     return RSC_OK;
+}
+static void pulse_formed(rsc_worker *w, int slot) {
+    w->pulse_at = slot;
+    w->pulse = w->pulse_ring + (size_t)slot * w->G;
 }
 
 /* Make the worker's stream wait for a pending remap into LES slot `slot`. */
@@ -1741,8 +1760,10 @@ int rsc_make_pulse(rsc_worker *w, const float sim_desc[16]) {
     s = pulse_geometry(w, mode, pulse_path(P, mode), P.mom_n, &grid, &threads, &smem);
     if (s) return s;
     if (pulse_path(P, mode) == 5) grid = std::min(grid, node_grid(P.n, threads));
-    s = pulse_d2h_wait(w);
+    int slot = 0;
+    s = pulse_slot(w, &slot);
     if (s) return s;
+    P.pulse = w->pulse_ring + (size_t)slot * w->G;
     if (w->pend && mode != RSC_PULSE_F64) {
         /* the recorded advance and this pulse in one pass over the state */
         int sgrid = 0;
@@ -1755,6 +1776,7 @@ int rsc_make_pulse(rsc_worker *w, const float sim_desc[16]) {
             rsc::k_step<1><<<sgrid, rsc::kAdvanceThreads, ssmem, w->stream>>>(w->pend_a, P, w->pend_blocks);
         }
         RSC_CUDA(cudaGetLastError());
+        pulse_formed(w, slot);
         w->pend = false;
         w->launches++;
         s = mark_read(w);
@@ -1772,6 +1794,7 @@ int rsc_make_pulse(rsc_worker *w, const float sim_desc[16]) {
     if (s) return s;
     launch_pulse(mode, P, grid, threads, smem, w->stream);
     RSC_CUDA(cudaGetLastError());
+    pulse_formed(w, slot);
     w->launches++;
     s = mark_read(w);
     if (s) return s;
@@ -1802,13 +1825,13 @@ int rsc_download_pulse_async(rsc_worker *w, float *pulse4) {
     if (w->d2h == nullptr) {
         RSC_CUDA(cudaStreamCreateWithFlags(&w->d2h, cudaStreamNonBlocking));
         RSC_CUDA(cudaEventCreateWithFlags(&w->pulse_ev, cudaEventDisableTiming));
-        RSC_CUDA(cudaEventCreateWithFlags(&w->d2h_done, cudaEventDisableTiming));
+        for (cudaEvent_t &e : w->d2h_done) RSC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     RSC_CUDA(cudaEventRecord(w->pulse_ev, w->stream));
     RSC_CUDA(cudaStreamWaitEvent(w->d2h, w->pulse_ev, 0));
     RSC_CUDA(cudaMemcpyAsync(pulse4, w->pulse, w->G * sizeof(float4), cudaMemcpyDeviceToHost, w->d2h));
-    RSC_CUDA(cudaEventRecord(w->d2h_done, w->d2h));
-    w->d2h_pending = true;
+    RSC_CUDA(cudaEventRecord(w->d2h_done[w->pulse_at], w->d2h));
+    w->d2h_busy[w->pulse_at] = true;
     return RSC_OK;
 }
 
@@ -1820,7 +1843,7 @@ int rsc_synchronize(rsc_worker *w) {
     if (s) return s;
     RSC_CUDA(cudaStreamSynchronize(w->stream));
     if (w->d2h) RSC_CUDA(cudaStreamSynchronize(w->d2h));
-    w->d2h_pending = false;
+    for (bool &b : w->d2h_busy) b = false;
     return RSC_OK;
 }
 
@@ -2354,8 +2377,10 @@ int rsc_autotune(rsc_worker *w, const float sim_desc[16], int *warps_out, int *b
     }
     P.materialize = 0;
     if (mode != RSC_PULSE_F64) use_nodes(w, P, mode);
-    s = pulse_d2h_wait(w);
+    int slot = 0;
+    s = pulse_slot(w, &slot);
     if (s) return s;
+    P.pulse = w->pulse_ring + (size_t)slot * w->G;
     EventPair ev;
     RSC_CUDA(ev.init());
     float best = INFINITY;
@@ -2385,6 +2410,7 @@ int rsc_autotune(rsc_worker *w, const float sim_desc[16], int *warps_out, int *b
             }
         }
     }
+    pulse_formed(w, slot);
     s = mark_read(w);
     if (s) return s;
     w->tune_warps = best_w;
