@@ -1937,6 +1937,7 @@ struct rsc_batch {
      * (0: as many as fit) */
     int adv_threads = rsc::kAdvanceThreads, adv_per_sm = 0;
     size_t adv_smem = 0;
+    int rain_form = 0;           /* what its kernel is compiled for: rain_kernel */
     bool nodes = false; /* the pulse through the node sums */
     bool tri = false;   /* the pulse kernel with the triangle range weight compiled in */
     /* per-instance launch descriptors and block prefixes */
@@ -2037,7 +2038,7 @@ int batch_prepare(rsc_batch *b, const rsc::BatchStep *row) {
     b->concept.assign(n, 0u);
     unsigned acc_r = 0, acc_d = 0, acc_p = 0;
     bool nodes = true;
-    int max_n = 0;
+    int max_n = 0, form = -1;
     for (size_t i = 0; i < n; i++) {
         rsc_worker *x = b->w[i];
         if (x->pos == nullptr) return fail(RSC_ERR_STATE, "instance %zu is not allocated", i);
@@ -2060,6 +2061,10 @@ int batch_prepare(rsc_batch *b, const rsc::BatchStep *row) {
         }
         b->h_rain_prefix[i] = acc_r;
         acc_r += (unsigned)((A.a.rain_count + (unsigned long long)b->adv_threads - 1) / (unsigned long long)b->adv_threads);
+        if (A.a.rain_count) {
+            const int f = A.a.rain_mode == 2 ? 0 : 1 + 2 * A.a.rain_mode + (rsm_f2u(A.a.wind[7]) == 7u ? 1 : 0);
+            form = form < 0 || form == f ? f : 0;
+        }
         b->h_deb_prefix[i] = acc_d;
         acc_d += blocks - A.a.rain_blocks;
         PulseArgs &P = b->h_pulse[i];
@@ -2106,10 +2111,11 @@ int batch_prepare(rsc_batch *b, const rsc::BatchStep *row) {
     b->h_deb_prefix[n] = acc_d;
     b->h_pulse_prefix[n] = acc_p;
     if (acc_r != b->rain_blocks || acc_d != b->deb_blocks || acc_p != b->pulse_blocks || threads != b->pulse_threads ||
-        smem != b->pulse_smem || tri != b->tri || nodes != b->nodes) {
+        smem != b->pulse_smem || tri != b->tri || nodes != b->nodes || std::max(form, 0) != b->rain_form) {
         batch_drop_graph(b);
     }
     b->tri = tri;
+    b->rain_form = std::max(form, 0);
     b->nodes = nodes;
     b->rain_blocks = acc_r;
     b->deb_blocks = acc_d;
@@ -2160,19 +2166,30 @@ cudaError_t batch_launch_pulse(rsc_batch *b, int k) {
  * k for the pulse of step k - 1 (which read the pair it overwrites).  The
  * advance stream starts after the work queued on the batch's stream and the
  * batch's stream ends after it. */
+/* The batched background advance's kernel for blocks of `threads`: compiled
+ * for the concept and LES spacing that all instances with drops share (form
+ * 1 + 2 mode + stretched, batch_prepare), 0 for a mixture and for fp_atts. */
+using RainKernel = void (*)(const rsc::BatchAdvance *, const rsc::BatchStep *, const unsigned *, int);
+template <int T>
+RainKernel rain_kernel_t(int form) {
+    switch (form) {
+        case 1: return rsc::k_advance_batch_rain<T, 0, -1>;
+        case 2: return rsc::k_advance_batch_rain<T, 0, 7>;
+        case 3: return rsc::k_advance_batch_rain<T, 1, -1>;
+        case 4: return rsc::k_advance_batch_rain<T, 1, 7>;
+        default: return rsc::k_advance_batch_rain<T>;
+    }
+}
+constexpr int kRainForms = 5;
+RainKernel rain_kernel(int threads, int form) {
+    return threads == 64 ? rain_kernel_t<64>(form) : (threads == 256 ? rain_kernel_t<256>(form) : rain_kernel_t<128>(form));
+}
+
 /* The background advance of one step of every instance at the batch's
  * advance shape. */
 cudaError_t batch_launch_rain(rsc_batch *b, const rsc::BatchAdvance *adv, const rsc::BatchStep *st) {
-    const int n = (int)b->w.size();
-    const unsigned g = b->rain_blocks;
-    const size_t sm = b->adv_smem;
-    if (b->adv_threads == 64) {
-        rsc::k_advance_batch_rain<64><<<g, 64, sm, b->adv>>>(adv, st, b->d_rain_prefix, n);
-    } else if (b->adv_threads == 256) {
-        rsc::k_advance_batch_rain<256><<<g, 256, sm, b->adv>>>(adv, st, b->d_rain_prefix, n);
-    } else {
-        rsc::k_advance_batch_rain<128><<<g, 128, sm, b->adv>>>(adv, st, b->d_rain_prefix, n);
-    }
+    rain_kernel(b->adv_threads, b->rain_form)<<<b->rain_blocks, (unsigned)b->adv_threads, b->adv_smem, b->adv>>>(
+        adv, st, b->d_rain_prefix, (int)b->w.size());
     return cudaGetLastError();
 }
 
@@ -2188,10 +2205,9 @@ int batch_advance_smem(rsc_batch *b, int threads, int per_sm, size_t *smem) {
     size_t want = (size_t)sm_bytes / (size_t)per_sm + 1;
     want = (want + 127) & ~(size_t)127;
     if (want > (size_t)optin - 1024) want = (size_t)optin - 1024;
-    void *k = threads == 64 ? reinterpret_cast<void *>(rsc::k_advance_batch_rain<64>)
-                            : (threads == 256 ? reinterpret_cast<void *>(rsc::k_advance_batch_rain<256>)
-                                              : reinterpret_cast<void *>(rsc::k_advance_batch_rain<128>));
-    RSC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want));
+    for (int form = 0; form < kRainForms; form++) {
+        RSC_CUDA(cudaFuncSetAttribute(rain_kernel(threads, form), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want));
+    }
     *smem = want;
     (void)b;
     return RSC_OK;

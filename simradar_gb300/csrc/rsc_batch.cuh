@@ -90,27 +90,50 @@ __device__ __forceinline__ int batch_advance_args(AdvanceArgs &sa, int &s_i, con
 }
 
 /* The background range of every instance (prefix over their background
- * blocks of T threads); the rain body chosen per instance by its concept.
- * A full SM of resident threads (32 registers) measured 6% faster per
- * batched step than 6 blocks of 256 (40 registers), which had been faster
- * than 5: resident warps hide the texel loads' latency.  T (64, 128, 256)
- * and the resident blocks per SM (limited through dynamic shared memory)
- * are the batch's advance shape, which rsc_batch_autotune times. */
-template <int T>
+ * blocks of T threads).  MODE and SP are compiled in when every instance's
+ * concept and LES spacing agree; -1 chooses per instance.  What bounds it is
+ * latency: the descriptor, the state, then the texels, so the descriptor's
+ * part of that chain is short (every thread finds the instance itself, only
+ * what a background step reads is copied, 0.4 of 2.5 KB, one barrier less)
+ * and the resident warps are many: a full SM of threads at 32 registers,
+ * although MODE 1 spills 52 bytes there, measured 6% faster per batched step
+ * than 6 blocks of 256 (40 registers).  12 instances of 65,536 to 1,048,576:
+ * 187 -> 175 us a step; one of 33.5M: 1727 -> 1667.  Two and four scatterers
+ * per thread, one after the other: 187 and 189, since the loop keeps the
+ * descriptor in registers and spills more.
+ * T (64, 128, 256) and the resident blocks per SM (limited through dynamic
+ * shared memory) are the batch's advance shape, which rsc_batch_autotune
+ * times. */
+template <int T, int MODE = -1, int SP = -1>
 __global__ void __launch_bounds__(T, 2048 / T)
 k_advance_batch_rain(const BatchAdvance *inst, const BatchStep *steps, const unsigned *prefix, int ninst) {
-    __shared__ __align__(16) AdvanceArgs sa;
-    __shared__ int s_i;
-    const int i = batch_advance_args(sa, s_i, inst, steps, prefix, ninst);
+    __shared__ __align__(16) RainArgs sa;
+    const int i = batch_instance(prefix, ninst, blockIdx.x);
+    const BatchAdvance &I = inst[i];
+    const BatchStep &S = steps[i];
+    const int les = S.les_id & 1;
+    block_copy(&sa, static_cast<const RainArgs *>(&I.a), sizeof(RainArgs));
+    __syncthreads();
+    if (threadIdx.x < 16) sa.sim[threadIdx.x] = S.sim[threadIdx.x];
+    if (threadIdx.x == 32) {
+        sa.uvwt = I.uvwt[les];
+        if (MODE < 0) sa.cpxx = I.cpxx[les];   /* read by fp_atts */
+        sa.pos_in = S.pos_r;
+        sa.rcs_in = S.rcs_r;
+        sa.pos = S.pos_w;
+        sa.rcs = S.rcs_w;
+    }
+    __syncthreads();
     const unsigned long long j = (unsigned long long)(blockIdx.x - __ldg(prefix + i)) * T + threadIdx.x;
     if (j >= sa.rain_count) return;
     const size_t x = (size_t)(sa.rain_origin + j);
     float4 pos, rcs;
     bool known;
-    if (sa.rain_mode == 1) {
-        rain_el(sa, x, pos, rcs, known);
-    } else if (sa.rain_mode == 0) {
-        rain_bg(sa, x, pos, rcs, known);
+    const int mode = MODE >= 0 ? MODE : sa.rain_mode;
+    if (mode == 1) {
+        rain_el<SP>(sa, x, pos, rcs, known);
+    } else if (mode == 0) {
+        rain_bg<SP>(sa, x, pos, rcs, known);
     } else {
         rain_fp(sa, x, pos, rcs, known);
     }

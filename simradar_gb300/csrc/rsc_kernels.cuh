@@ -31,12 +31,13 @@ struct DebrisType {
     float rcs[16];
 };
 
-struct AdvanceArgs {
+/* What a background step reads. */
+struct RainArgs {
     /* pos and rcs are read from pos_in / rcs_in and written to pos / rcs:
      * the same arrays in place, or the worker's second pair so that the
      * pulse of the same step can read the first pair meanwhile */
     const float4 *pos_in, *rcs_in;
-    float4 *pos, *vel, *ori, *tum, *rcs;
+    float4 *pos, *vel, *rcs;
     uint4 *rnd;
     PairImage uvwt;
     Image cpxx;
@@ -44,10 +45,14 @@ struct AdvanceArgs {
     float sim[16];
     const float4 *drop;
     float drop_desc[4];
-    const float *dff;
-    float dff_desc[16];
     unsigned long long rain_origin, rain_count;
     int rain_mode; /* 0 bg_atts, 1 el_atts, 2 fp_atts */
+};
+
+struct AdvanceArgs : RainArgs {
+    float4 *ori, *tum;
+    const float *dff;
+    float dff_desc[16];
     unsigned rain_blocks;
     int ntypes;
     unsigned long long deb_prefix[RSC_MAX_TYPES]; /* cumulative debris counts */
@@ -64,7 +69,7 @@ struct RainNext {
     bool respawn;
 };
 
-__device__ __forceinline__ void rain_store(const AdvanceArgs &a, size_t i, const RainNext &o) {
+__device__ __forceinline__ void rain_store(const RainArgs &a, size_t i, const RainNext &o) {
     a.pos[i] = o.pos;
     a.vel[i] = o.vel;
     if (o.respawn) {
@@ -78,7 +83,7 @@ __device__ __forceinline__ void rain_store(const AdvanceArgs &a, size_t i, const
 
 /* respawn (rs.cl:546-556, rs.cl:668-678): the only time the seed is read */
 template <bool FMA>
-__device__ __forceinline__ void rain_respawn(const AdvanceArgs &a, size_t i, const float *sd, RainNext &o) {
+__device__ __forceinline__ void rain_respawn(const RainArgs &a, size_t i, const float *sd, RainNext &o) {
     uint4 seed = a.rnd[i];
     float4 r = cl_rand(&seed);
     if (FMA) {
@@ -98,7 +103,7 @@ __device__ __forceinline__ void rain_respawn(const AdvanceArgs &a, size_t i, con
 
 /* ---- el_atts (rs.cl:653-739) ---- */
 template <int SP = -1>
-__device__ __forceinline__ void rain_el_next(const AdvanceArgs &a, size_t i, RainNext &o) {
+__device__ __forceinline__ void rain_el_next(const RainArgs &a, size_t i, RainNext &o) {
     const float *sd = a.sim;
     const float dt = sd[11];
     const uint32_t concept = __float_as_uint(sd[5]);
@@ -148,7 +153,7 @@ __device__ __forceinline__ void rain_el_next(const AdvanceArgs &a, size_t i, Rai
 
 /* ---- bg_atts (rs.cl:533-580) ---- */
 template <int SP = -1>
-__device__ __forceinline__ void rain_bg_next(const AdvanceArgs &a, size_t i, RainNext &o) {
+__device__ __forceinline__ void rain_bg_next(const RainArgs &a, size_t i, RainNext &o) {
     const float *sd = a.sim;
     const float dt = sd[11];
     float4 pos = a.pos_in[i];
@@ -170,7 +175,7 @@ __device__ __forceinline__ void rain_bg_next(const AdvanceArgs &a, size_t i, Rai
 /* The background step of scatterer i, stored; its new position and
  * backscatter returned (xk false on a respawn, where xo is the kept one). */
 template <int SP = -1>
-__device__ __forceinline__ void rain_el(const AdvanceArgs &a, size_t i, float4 &po, float4 &xo, bool &xk) {
+__device__ __forceinline__ void rain_el(const RainArgs &a, size_t i, float4 &po, float4 &xo, bool &xk) {
     RainNext o;
     rain_el_next<SP>(a, i, o);
     rain_store(a, i, o);
@@ -180,7 +185,7 @@ __device__ __forceinline__ void rain_el(const AdvanceArgs &a, size_t i, float4 &
 }
 
 template <int SP = -1>
-__device__ __forceinline__ void rain_bg(const AdvanceArgs &a, size_t i, float4 &po, float4 &xo, bool &xk) {
+__device__ __forceinline__ void rain_bg(const RainArgs &a, size_t i, float4 &po, float4 &xo, bool &xk) {
     RainNext o;
     rain_bg_next<SP>(a, i, o);
     rain_store(a, i, o);
@@ -190,7 +195,7 @@ __device__ __forceinline__ void rain_bg(const AdvanceArgs &a, size_t i, float4 &
 }
 
 /* ---- fp_atts (rs.cl:590-648) ---- */
-__device__ __forceinline__ void rain_fp(const AdvanceArgs &a, size_t i, float4 &po, float4 &xo, bool &xk) {
+__device__ __forceinline__ void rain_fp(const RainArgs &a, size_t i, float4 &po, float4 &xo, bool &xk) {
     const float *sd = a.sim;
     const float wav_num = sd[4];
     const float dt = sd[11];
