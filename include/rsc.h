@@ -448,7 +448,7 @@ int rsc_les_close(rsc_les_source *src);
 const char *rsc_les_last_error(void);
 
 /* Limits of rsc_make_pulse_noalloc (its scratch is a fixed device array of
- * about 9 KB per GPU that loads this library). */
+ * about 18 KB per GPU that loads this library). */
 #define RSC_NOALLOC_MAX_GATES 128
 #define RSC_NOALLOC_MAX_RANGE_TABLE 64
 #define RSC_NOALLOC_MAX_ANGULAR_TABLE 1024
@@ -472,7 +472,7 @@ const char *rsc_les_last_error(void);
  * The scratch the kernels need (an FP64 accumulator per gate, a completion
  * counter, gate origins, the weight tables) lives in one fixed __device__
  * array in the library instead of in memory the call allocates: every GPU
- * that loads the library holds about 9 KB for it until the process exits.
+ * that loads the library holds about 18 KB for it until the process exits.
  * The accumulator and the counter are cleared at each call.  The first call
  * on a device looks the array's address up (once per device, with that
  * device current); make that first call before any stream capture.  All

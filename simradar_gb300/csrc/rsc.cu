@@ -473,6 +473,7 @@ typedef void (*PulseKernel)(const PulseArgs);
  * the path at run time (one compensated kernel per path measured 7% slower). */
 PulseKernel pulse_kernel(int mode, int path) {
     if (mode == RSC_PULSE_PLAIN) {
+        if (path == 6) return rsc::k_pulse_nodes_any;
         if (path == 5) return rsc::k_pulse_nodes;
         if (path == 4) return rsc::k_pulse_group<0, kPulseGroup, 1>;
         if (path == 3) return rsc::k_pulse_group<0, kPulseGroup>;
@@ -489,9 +490,9 @@ PulseKernel pulse_kernel(int mode, int path) {
 /* 0 atomics, 1 coherent warps, 2 every gate, 3 coherent warps with
  * kPulseGroup scatterers per lane (the compensated form, and the plain form
  * when it does not write aux / sig), 4 the same with the triangle range
- * table compiled in */
+ * table compiled in, 5 node sums, 6 node sums scatterer by scatterer */
 int pulse_path(const PulseArgs &P, int mode) {
-    if (mode != RSC_PULSE_F64 && P.mom_n > 0) return 5;
+    if (mode != RSC_PULSE_F64 && P.mom_n > 0) return P.any ? 6 : 5;
     if (P.dense) return 2;
     if (P.coherent_span <= 0) return 0;
     if ((mode == RSC_PULSE_PLAIN && !P.materialize) || mode == RSC_PULSE_COMPENSATED) return P.rw_tri ? 4 : 3;
@@ -502,6 +503,7 @@ int pulse_path(const PulseArgs &P, int mode) {
  * the advance of the same step its share of the SM (README scale, a dwell of
  * 10 pulses: 580 us with 3, 592 with 4, 588 with 2). */
 constexpr int kNodePerSm = 3;
+constexpr int kNodeAnyPerSm = 4;
 
 /* Launch shape of the pulse kernel (one-instance or batched form) for G
  * gates: warps per block as many as fit 200 KB of bins (at most 16, at most
@@ -509,17 +511,18 @@ constexpr int kNodePerSm = 3;
  * calculator (at most 4, at most want_per_sm when that is > 0). */
 int pulse_shape(int mode, bool batch, uint32_t G, int want_warps, int want_per_sm, int *per_sm_out, int *threads,
                 size_t *smem, int path = 0, int mom_n = 0) {
-    if (path == 5) {
+    if (path == 5 || path == 6) {
         const int warps = rsc::kNodeThreads / 32;
         *threads = 32 * (want_warps > 0 && want_warps < warps ? want_warps : warps);
-        *smem = rsc::node_smem_bytes(G, mom_n, mode == RSC_PULSE_COMPENSATED);
+        *smem = path == 6 ? rsc::node_any_smem_bytes(G, mom_n, *threads / 32)
+                          : rsc::node_smem_bytes(G, mom_n, mode == RSC_PULSE_COMPENSATED);
         int fit = 1;
         cudaError_t e = !batch ? kernel_occupancy(pulse_kernel(mode, path), *threads, *smem, &fit)
                         : mode == RSC_PULSE_PLAIN
                             ? kernel_occupancy(rsc::k_pulse_batch_nodes<0>, *threads, *smem, &fit)
                             : kernel_occupancy(rsc::k_pulse_batch_nodes<1>, *threads, *smem, &fit);
         if (e != cudaSuccess) return cuda_fail(RSC_ERR_CUDA, "pulse kernel configuration: %s", cudaGetErrorString(e));
-        if (want_per_sm <= 0) want_per_sm = kNodePerSm;
+        if (want_per_sm <= 0) want_per_sm = path == 6 ? kNodeAnyPerSm : kNodePerSm;
         if (fit < 1) fit = 1;
         if (want_per_sm < fit) fit = want_per_sm;
         *per_sm_out = fit;
@@ -679,10 +682,21 @@ double window_margin(double drift, float range_start, float range_delta, uint32_
 
 /* A pulse through the node sums where the triangle allows them: compensated
  * always (unless rsc_set_pulse_moments turned them off), plain on a state in
- * spatial order or with a triangle too wide for the gate window. */
-void use_nodes(rsc_worker *w, PulseArgs &P, int mode) {
+ * spatial order, scatterer by scatterer on one in the caller's order
+ * when the triangle is wide enough for that (kNodeAnyLeast) and the warps'
+ * sums fit (kNodeAnyMost).  Beyond, and in a batch, whose instances share one
+ * kernel, only with a triangle too wide for the gate window. */
+void use_nodes(rsc_worker *w, PulseArgs &P, int mode, bool batch) {
     const int n = node_span(P);
-    if (mode == RSC_PULSE_PLAIN ? n == 0 || (P.coherent_span <= 0 && !P.dense) : n == 0 || !w->moments) return;
+    if (n == 0 || (mode != RSC_PULSE_PLAIN && !w->moments)) return;
+    if (mode == RSC_PULSE_PLAIN && P.coherent_span <= 0) {
+        if (!batch && n >= rsc::kNodeAnyLeast &&
+            rsc::node_any_smem_bytes(w->G, n, rsc::kNodeThreads / 32) <= rsc::kNodeAnyMost) {
+            P.any = 1;
+        } else if (!P.dense) {
+            return;
+        }
+    }
     P.mom_n = n;
     P.node = w->node + (rsc::kNodeMaxN - n);
     P.stray = reinterpret_cast<float4 *>(w->acc64 + (2 * rsc::node_count(w->G, rsc::kNodeMaxN) + w->G) * 4);
@@ -1756,12 +1770,12 @@ int rsc_make_pulse(rsc_worker *w, const float sim_desc[16]) {
     }
     const bool mat = (mode == RSC_PULSE_PLAIN) && (w->materialize || sim_desc[15] != 0.0f);
     P.materialize = mat ? 1 : 0;
-    if (mode != RSC_PULSE_F64 && !mat && !w->pend) use_nodes(w, P, mode);
+    if (mode != RSC_PULSE_F64 && !mat && !w->pend) use_nodes(w, P, mode, false);
     int grid = 0, threads = 0;
     size_t smem = 0;
     s = pulse_geometry(w, mode, pulse_path(P, mode), P.mom_n, &grid, &threads, &smem);
     if (s) return s;
-    if (pulse_path(P, mode) == 5) grid = std::min(grid, node_grid(P.n, threads));
+    if (pulse_path(P, mode) >= 5) grid = std::min(grid, node_grid(P.n, threads));
     int slot = 0;
     s = pulse_slot(w, &slot);
     if (s) return s;
@@ -2077,7 +2091,7 @@ int batch_prepare(rsc_batch *b, const rsc::BatchStep *row) {
             P.runs = x->runs;
         }
         P.materialize = 0;
-        if (b->mode != RSC_PULSE_F64 && !b->persist) use_nodes(x, P, b->mode);
+        if (b->mode != RSC_PULSE_F64 && !b->persist) use_nodes(x, P, b->mode, true);
         nodes = nodes && P.mom_n > 0;
         max_n = std::max(max_n, P.mom_n);
         tri = tri && P.rw_tri;
@@ -2394,7 +2408,7 @@ int rsc_autotune(rsc_worker *w, const float sim_desc[16], int *warps_out, int *b
         P.runs = w->runs;
     }
     P.materialize = 0;
-    if (mode != RSC_PULSE_F64) use_nodes(w, P, mode);
+    if (mode != RSC_PULSE_F64) use_nodes(w, P, mode, false);
     int slot = 0;
     s = pulse_slot(w, &slot);
     if (s) return s;
@@ -3096,14 +3110,16 @@ int rsc_batch_get_shape(rsc_batch *b, int *warps, int *blocks_per_sm) {
 
 /* ---- pulse formation that allocates nothing ---------------------------------
  * The pulse kernel needs scratch memory beyond its inputs and outputs: an FP64
- * accumulator per gate and lane, a completion counter, and the gate origins
- * and weight tables in device memory.  rsc_make_pulse takes them from buffers
+ * accumulator per gate (and node of the gate grid) and lane, a completion
+ * counter, and the gate origins, nodes and weight tables in device memory.  rsc_make_pulse takes them from buffers
  * rsc_worker_malloc allocated.  rsc_make_pulse_noalloc takes them from the
  * fixed array below instead, so a caller that must not allocate device memory
  * can still form a pulse from its own device buffers. */
 #define RSC_NA_ACC_OFF 0
-#define RSC_NA_ACC_BYTES ((size_t)RSC_NOALLOC_MAX_GATES * 4 * sizeof(double))
-#define RSC_NA_RK_OFF (RSC_NA_ACC_OFF + RSC_NA_ACC_BYTES)
+#define RSC_NA_NODES ((size_t)RSC_NOALLOC_MAX_GATES + 2 * rsc::kNodeMaxN)
+#define RSC_NA_ACC_BYTES ((RSC_NA_NODES + RSC_NOALLOC_MAX_GATES) * 4 * sizeof(double))
+#define RSC_NA_NODE_OFF (RSC_NA_ACC_OFF + RSC_NA_ACC_BYTES)
+#define RSC_NA_RK_OFF (RSC_NA_NODE_OFF + RSC_NA_NODES * 4)
 #define RSC_NA_RW_OFF (RSC_NA_RK_OFF + (size_t)RSC_NOALLOC_MAX_GATES * 4)
 #define RSC_NA_AW_OFF (RSC_NA_RW_OFF + (size_t)RSC_NOALLOC_MAX_RANGE_TABLE * 4)
 #define RSC_NA_COUNTER_OFF (RSC_NA_AW_OFF + (size_t)RSC_NOALLOC_MAX_ANGULAR_TABLE * 4)
@@ -3146,12 +3162,13 @@ struct NoAllocSetup {
     float rw[RSC_NOALLOC_MAX_RANGE_TABLE];
     float aw[RSC_NOALLOC_MAX_ANGULAR_TABLE];
     uint32_t rw_n, aw_n, G;
+    int n;                  /* half width of the triangle in gates for the node sums, 0 without them */
     float range_start, range_delta;
     unsigned char *scratch;
 };
 
 /* Fill the scratch: the weight tables, the gate origins as the FP32 running
- * sum of make_pulse_pass_1 (rs.cl:1214), and a zero accumulator and counter
+ * sum of make_pulse_pass_1 (rs.cl:1214), the nodes, and a zero accumulator and counter
  * (the pulse kernel leaves both at zero, but a launch that failed part way
  * might not have).  One block. */
 __global__ void __launch_bounds__(256) k_noalloc_setup(const NoAllocSetup a) {
@@ -3161,14 +3178,24 @@ __global__ void __launch_bounds__(256) k_noalloc_setup(const NoAllocSetup a) {
     double *acc = reinterpret_cast<double *>(a.scratch + RSC_NA_ACC_OFF);
     for (uint32_t i = threadIdx.x; i < a.rw_n; i += blockDim.x) rw[i] = a.rw[i];
     for (uint32_t i = threadIdx.x; i < a.aw_n; i += blockDim.x) aw[i] = a.aw[i];
-    for (uint32_t i = threadIdx.x; i < 4 * a.G; i += blockDim.x) acc[i] = 0.0;
+    const uint32_t nodes = a.n > 0 ? rsc::node_count(a.G, a.n) : 0u;
+    for (uint32_t i = threadIdx.x; i < 4 * (nodes + a.G); i += blockDim.x) acc[i] = 0.0;
+    __shared__ float origin[RSC_NOALLOC_MAX_GATES];
     if (threadIdx.x == 0) {
         float r = a.range_start;
         for (uint32_t k = 0; k < a.G; k++) {
-            rk[k] = r;
+            origin[k] = r;
             r = r + a.range_delta;
         }
         *reinterpret_cast<unsigned *>(a.scratch + RSC_NA_COUNTER_OFF) = 0u;
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < a.G; k += blockDim.x) rk[k] = origin[k];
+    /* the nodes, as set_gates forms them */
+    float *node = reinterpret_cast<float *>(a.scratch + RSC_NA_NODE_OFF);
+    for (uint32_t i = threadIdx.x; i < nodes; i += blockDim.x) {
+        const int m = (int)i - a.n, k = min(max(m, 0), (int)a.G - 1);
+        node[i] = (float)((double)origin[k] + (double)(m - k) * (double)a.range_delta);
     }
 }
 
@@ -3262,11 +3289,28 @@ int rsc_make_pulse_noalloc(const float *pos4, const float *rcs4, size_t num_scat
             P.win_hi = (float)hi;
         }
     }
-    /* launch geometry of the plain pulse kernel */
-    const PulseKernel kern = pulse_kernel(RSC_PULSE_PLAIN, pulse_path(P, RSC_PULSE_PLAIN));
     int dev = 0, sms = 0, per_sm = 1;
     RSC_CUDA(cudaGetDevice(&dev));
     RSC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    /* scatterer by scatterer onto the nodes where the triangle allows it: 48 KB
+     * hold the sums of any G here, so the launch needs no query */
+    setup.n = node_span(P);
+    if (setup.n < rsc::kNodeAnyLeast) setup.n = 0;
+    if (setup.n > 0) {
+        P.mom_n = setup.n;
+        P.any = 1;
+        P.node = reinterpret_cast<const float *>(b + RSC_NA_NODE_OFF);
+        const size_t bytes = rsc::node_any_smem_bytes(G, setup.n, rsc::kNodeThreads / 32);
+        static_assert(RSC_NA_NODES * (1 + 4 * (rsc::kNodeThreads / 32)) * sizeof(float) <= 47 * 1024, "node sums");
+        const int blocks = std::min(sms * kNodeAnyPerSm, node_grid(num_scats, rsc::kNodeThreads));
+        k_noalloc_setup<<<1, 256, 0, st>>>(setup);
+        RSC_CUDA(cudaGetLastError());
+        rsc::k_pulse_nodes_any<<<blocks, rsc::kNodeThreads, bytes, st>>>(P);
+        RSC_CUDA(cudaGetLastError());
+        return RSC_OK;
+    }
+    /* launch geometry of the plain pulse kernel */
+    const PulseKernel kern = pulse_kernel(RSC_PULSE_PLAIN, pulse_path(P, RSC_PULSE_PLAIN));
     const int threads = 16 * 32;
     const size_t smem = 16 * rsc::pulse_warp_bytes(RSC_PULSE_PLAIN, G) + 2 * G * sizeof(float);
     RSC_CUDA(kernel_occupancy(kern, threads, smem, &per_sm));

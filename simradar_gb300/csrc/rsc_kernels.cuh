@@ -481,8 +481,10 @@ struct PulseArgs {
     int dense;
     int coherent_span;   /* warp-coherent gate path when a warp spans fewer gates */
     int materialize;
-    int mom_n;           /* compensated form on the triangle whose support is mom_n gate spacings: terms
-                          * summed per range interval as moments (PulseBins::add_k), 0 otherwise */
+    int mom_n;           /* triangle whose half width is mom_n gate spacings: sums on the gate grid's nodes
+                          * (rsc_nodes.cuh) or, compensated in the batch's other forms, moments per range
+                          * interval (PulseBins::add_k); 0 gate by gate */
+    int any;             /* node sums scatterer by scatterer: a state in the caller's order */
     double *acc64;       /* G * 4 FP64 accumulators, zero between launches */
     unsigned *counter;
     const float *node;          /* node positions of the gate grid, index 0 at node -mom_n (rsc_nodes.cuh) */

@@ -544,23 +544,17 @@ __device__ __forceinline__ void node_settle(const PulseArgs &P, NodeWindow &W, c
     }
 }
 
-/* The block's node sums into the grid's accumulator, the last block forming
- * the gates and leaving accumulator and counter at zero.  A chain of round
- * trips to L2 at the end of every pulse: the sums (reductions nothing waits
- * for), the ticket, the loads, all of them before the first gate is formed
- * (393,225 scatterers: 333.5 -> 328.5 us for 10 steps; 500,000 on gates 2.5 m
- * apart: 140 -> 137.7 for 4, against generic atomics, a fence on both sides
- * of the ticket and the gates' own sums loaded one by one). */
-template <int MODE>
-__device__ __forceinline__ void node_finish(const PulseArgs &P, double *bins, unsigned nblk) {
+/* The end of a block whose sums are on their way to the grid's accumulator:
+ * the last block forms the gates and leaves accumulator and counter at zero.
+ * A chain of round trips to L2 at the end of every pulse: the sums
+ * (reductions nothing waits for), the ticket, the loads, all of them before
+ * the first gate is formed (393,225 scatterers: 333.5 -> 328.5 us for 10
+ * steps; 500,000 on gates 2.5 m apart: 140 -> 137.7 for 4, against generic
+ * atomics, a fence on both sides of the ticket and the gates' own sums loaded
+ * one by one).  STRAY: scatterers may have gone to P.stray. */
+template <int MODE, bool STRAY>
+__device__ __forceinline__ void node_gates(const PulseArgs &P, double *bins, unsigned nblk) {
     const unsigned nodes = node_count(P.G, P.mom_n), outs = P.G * 4;
-    if (MODE == 0) {
-        __syncthreads();
-        for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) {
-            const double v = bins[o];
-            if (v != 0.0) red_add(P.acc64 + o, v);
-        }
-    }
     __shared__ bool s_last;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -610,14 +604,14 @@ __device__ __forceinline__ void node_finish(const PulseArgs &P, double *bins, un
         float v = (float)__ldcg(P.acc64 + o), t = 0.0f;
 #pragma unroll
         for (unsigned c = 0; c < kNodeCopies; c++) {
-            if (c < copies) t = t + __ldcg(stray + (size_t)c * 4 * nodes + o);
+            if (STRAY && c < copies) t = t + __ldcg(stray + (size_t)c * 4 * nodes + o);
         }
         sums[o] = v + t;   /* over bins[o / 2], whose sums are out */
     }
     for (unsigned o = threadIdx.x; o < nodes; o += blockDim.x) at_node[o] = __ldg(P.node + o);
     __syncthreads();
     for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) P.acc64[o] = 0.0;
-    for (unsigned o = threadIdx.x; o < nodes * copies; o += blockDim.x) P.stray[o] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (unsigned o = threadIdx.x; STRAY && o < nodes * copies; o += blockDim.x) P.stray[o] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const int n = P.mom_n;
     for (unsigned o = threadIdx.x; o < outs; o += blockDim.x) {
         const unsigned k = o >> 2, l = o & 3u;
@@ -637,6 +631,20 @@ __device__ __forceinline__ void node_finish(const PulseArgs &P, double *bins, un
         reinterpret_cast<float *>(P.pulse)[o] = sum;
     }
     if (threadIdx.x == 0) *P.counter = 0u;
+}
+
+/* The block's node sums into the grid's accumulator, and the gates. */
+template <int MODE>
+__device__ __forceinline__ void node_finish(const PulseArgs &P, double *bins, unsigned nblk) {
+    if (MODE == 0) {
+        const unsigned nodes = node_count(P.G, P.mom_n);
+        __syncthreads();
+        for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) {
+            const double v = bins[o];
+            if (v != 0.0) red_add(P.acc64 + o, v);
+        }
+    }
+    node_gates<MODE, true>(P, bins, nblk);
 }
 
 /* A run of 64 into the warp's window. */
@@ -786,6 +794,87 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeMinBlocks) k_pulse_nodes(co
 
 __global__ void __launch_bounds__(kNodeThreads, kCompMinBlocks) k_pulse_nodes_comp(const PulseArgs P) {
     node_body<1>(P, blockIdx.x, gridDim.x);
+}
+
+/* ---- the plain form on a state in the caller's order ----
+ * No run lies together, so every scatterer goes to its two nodes by itself: 8
+ * additions to the warp's own node sums in shared memory, lane l's node next
+ * to the next lane's.  Bound by those additions (compare and swap, lane after
+ * lane where they meet), so fewer is faster: the gates' own sums take 4 for
+ * each gate a scatterer reaches, or a visit to every gate when the gate window
+ * does not hold them.  2,000,000 scatterers: n = 2 59 -> 41 us, n = 4 126 (as
+ * reductions in L2, which meet in a few addresses) -> 41; 300,000 from the
+ * caller's own buffers, n = 4 100 -> 27.  With 3 and 2 blocks per SM 43 and 56
+ * instead of 41. */
+__host__ __device__ __forceinline__ size_t node_any_smem_bytes(unsigned G, int n, int warps) {
+    return (size_t)node_count(G, n) * (1 + 4 * (size_t)warps) * sizeof(float);
+}
+/* ... while 4 blocks fit an SM with it. */
+constexpr size_t kNodeAnyMost = 54 * 1024;
+/* Narrower triangles reach two gates, whose own sums are as few (2,000,000:
+ * 41.5 us on the nodes, 41.3 there; 30,000: 10.5, 8.7). */
+constexpr int kNodeAnyLeast = 2;
+
+__device__ __forceinline__ void node_any_add(const PulseArgs &P, const float *E, int last, float *mine, unsigned nodes,
+                                             const float4 &p, const float4 &x) {
+    Sig g;
+    if (!signal_plain_mid(P, p, x, g)) {
+        Sig32 sg;
+        signal_plain(P, p, x, sg);
+        g.r = sg.r;
+#pragma unroll
+        for (int l = 0; l < 4; l++) g.s[l] = sg.s.v[l];
+    }
+    if (!sig_finite(g)) {
+        node_non_finite(P, g.r, g.s[0], g.s[1], g.s[2], g.s[3]);
+        return;
+    }
+    /* node_interval and node_stray, on the nodes in shared memory */
+    const float jf = floorf((g.r - E[0]) * P.inv_delta);
+    if (!(jf >= -1.0f && jf <= (float)(last + 1))) return;
+    int j = min(max((int)jf, 0), last);
+    if (g.r < E[j]) j--;
+    else if (g.r >= E[j + 1]) j++;
+    if (j < 0 || j > last) return;
+    const float a = E[j], b = E[j + 1], i = 1.0f / (b - a);
+    const float wa = (b - g.r) * i, wb = (g.r - a) * i;
+#pragma unroll
+    for (int l = 0; l < 4; l++) {
+        float *o = mine + (size_t)l * nodes + j;
+        atomicAdd(o, wa * g.s[l]);
+        atomicAdd(o + 1, wb * g.s[l]);
+    }
+}
+
+__global__ void __launch_bounds__(kNodeThreads, kNodeMinBlocks) k_pulse_nodes_any(const PulseArgs P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const unsigned nodes = node_count(P.G, P.mom_n), nwarps = blockDim.x >> 5, warp = threadIdx.x >> 5;
+    const unsigned lane = threadIdx.x & 31u;
+    float *E = reinterpret_cast<float *>(smem_raw), *sums = E + nodes, *mine = sums + (size_t)warp * 4 * nodes;
+    for (unsigned o = threadIdx.x; o < nodes; o += blockDim.x) E[o] = __ldg(P.node + o);
+    for (unsigned o = threadIdx.x; o < nwarps * 4 * nodes; o += blockDim.x) sums[o] = 0.0f;
+    __syncthreads();
+    const int last = (int)nodes - 2;
+    const unsigned long long n = P.n, stride = (unsigned long long)gridDim.x * blockDim.x * 2ull;
+    for (unsigned long long base = ((unsigned long long)blockIdx.x * nwarps + warp) * 64ull + lane; base < n; base += stride) {
+        const bool two = base + 32ull < n;
+        const float4 p0 = __ldg(P.pos + base), x0 = __ldg(P.rcs + base);
+        float4 p1 = p0, x1 = x0;
+        if (two) {
+            p1 = __ldg(P.pos + base + 32);
+            x1 = __ldg(P.rcs + base + 32);
+        }
+        node_any_add(P, E, last, mine, nodes, p0, x0);
+        if (two) node_any_add(P, E, last, mine, nodes, p1, x1);
+    }
+    __syncthreads();
+    for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) {
+        const unsigned at = (o & 3u) * nodes + (o >> 2);
+        float v = 0.0f;
+        for (unsigned w = 0; w < nwarps; w++) v = v + sums[(size_t)w * 4 * nodes + at];
+        if (v != 0.0f) red_add(P.acc64 + o, (double)v);
+    }
+    node_gates<0, false>(P, reinterpret_cast<double *>(smem_raw), gridDim.x);
 }
 
 }  // namespace rsc
