@@ -492,6 +492,7 @@ PulseKernel pulse_kernel(int mode, int path) {
  * when it does not write aux / sig), 4 the same with the triangle range
  * table compiled in, 5 node sums, 6 node sums scatterer by scatterer */
 int pulse_path(const PulseArgs &P, int mode) {
+    if (mode == RSC_PULSE_COMPENSATED && P.any) return 4;
     if (mode != RSC_PULSE_F64 && P.mom_n > 0) return P.any ? 6 : 5;
     if (P.dense) return 2;
     if (P.coherent_span <= 0) return 0;
@@ -680,27 +681,48 @@ double window_margin(double drift, float range_start, float range_delta, uint32_
     return (drift + 2.0 * ulp_r) / delta + 8.0 * ldexp(1.0, -23) * span + 1.0e-4;
 }
 
-/* A pulse through the node sums where the triangle allows them: compensated
- * always (unless rsc_set_pulse_moments turned them off), plain on a state in
- * spatial order, scatterer by scatterer on one in the caller's order
- * when the triangle is wide enough for that (kNodeAnyLeast) and the warps'
- * sums fit (kNodeAnyMost).  Beyond, and in a batch, whose instances share one
- * kernel, only with a triangle too wide for the gate window. */
+/* Advances after which a state that is no longer sorted counts as out of
+ * order: by then the drops respawned elsewhere, which go one by one, add up. */
+constexpr uint64_t kOrderedSteps = 2048;
+
+/* Gates from which compensated single scatterers meeting in L2 take less time
+ * than every gate visited: the one shrinks with the nodes (2 M scatterers on
+ * 77 gates 7.5 m apart 1875 us), the other grows with the gates (1670). */
+constexpr uint32_t kStrayGates = 82;
+
+/* A pulse through the node sums where the triangle allows them.
+ * On a state in spatial order always, unless rsc_set_pulse_moments turned the
+ * compensated ones off.  Out of it (before the first sort, after an upload)
+ * plain scatterer by scatterer when the triangle is wide enough for that
+ * (kNodeAnyLeast) and the warps' sums fit (kNodeAnyMost), and compensated by
+ * the warp's moments per interval: single scatterers would meet in L2 (first
+ * pulse of 8.4 M: 14 ms against 1).  Where neither serves, and in a batch,
+ * whose instances share one kernel, only with a triangle too wide for the gate
+ * window, whose other form visits every gate. */
 void use_nodes(rsc_worker *w, PulseArgs &P, int mode, bool batch) {
     const int n = node_span(P);
     if (n == 0 || (mode != RSC_PULSE_PLAIN && !w->moments)) return;
-    if (mode == RSC_PULSE_PLAIN && P.coherent_span <= 0) {
-        if (!batch && n >= rsc::kNodeAnyLeast &&
+    const bool ordered = w->perm != nullptr && !w->sort_due && w->since_sort < kOrderedSteps;
+    if (!ordered && mode == RSC_PULSE_PLAIN) {
+        if (!batch && P.coherent_span <= 0 && n >= rsc::kNodeAnyLeast &&
             rsc::node_any_smem_bytes(w->G, n, rsc::kNodeThreads / 32) <= rsc::kNodeAnyMost) {
             P.any = 1;
         } else if (!P.dense) {
             return;
         }
+    } else if (!ordered) {
+        const int m = moment_span(P);
+        if (m > 0) {
+            P.mom_n = batch ? 0 : m;
+            P.any = batch ? 0 : 1;
+            return;
+        }
+        if (w->G < kStrayGates) return;
     }
     P.mom_n = n;
     P.node = w->node + (rsc::kNodeMaxN - n);
     P.stray = reinterpret_cast<float4 *>(w->acc64 + (2 * rsc::node_count(w->G, rsc::kNodeMaxN) + w->G) * 4);
-    P.lead = w->perm != nullptr ? w->sort_end : 0;
+    P.lead = ordered ? w->sort_end : 0;
     /* half a gate more than the triangles reach; everything when an antenna
      * weight is not finite, which any range meets */
     const double lo = (double)w->range_start - (n + 0.5) * (double)w->range_delta;

@@ -484,7 +484,8 @@ struct PulseArgs {
     int mom_n;           /* triangle whose half width is mom_n gate spacings: sums on the gate grid's nodes
                           * (rsc_nodes.cuh) or, compensated in the batch's other forms, moments per range
                           * interval (PulseBins::add_k); 0 gate by gate */
-    int any;             /* node sums scatterer by scatterer: a state in the caller's order */
+    int any;             /* a state out of spatial order: plain, the node sums scatterer by scatterer;
+                          * compensated, the moments instead of the node sums */
     double *acc64;       /* G * 4 FP64 accumulators, zero between launches */
     unsigned *counter;
     const float *node;          /* node positions of the gate grid, index 0 at node -mom_n (rsc_nodes.cuh) */
