@@ -177,8 +177,8 @@ int rsc_set_materialize_sig_aux(rsc_worker *w, int enable);
 
 /* The compensated form's gate sums on the triangle range weight (additive,
  * default 1): 1 sums each scatterer's term into its one range interval as
- * two moments (the triangle is linear within an interval) and forms the
- * gates from them; 0 weighs every term into every gate it reaches.  Both
+ * two moments (the triangle is linear within an interval; about the interval's
+ * node on a state in spatial order) and forms the gates from them; 0 weighs every term into every gate it reaches.  Both
  * are error-free double-float sums; the pulses agree to the double-float's
  * precision.  Read by rsc_make_pulse and by a batch's runs. */
 int rsc_set_pulse_moments(rsc_worker *w, int enable);
@@ -196,9 +196,9 @@ int rsc_get_stream(rsc_worker *w, void **stream);
 int rsc_get_advance_stream(rsc_worker *w, void **stream);
 
 /* ---- spatial order (additive) ----
- * The worker keeps its background scatterers (type 0) in Morton order of
- * their cell in the scan box, restored by a counting sort after every
- * `steps` calls of rsc_advance_time (and after an upload of positions); 0
+ * The worker keeps the scatterers of every type (of type 0 alone when the
+ * types' ranges do not follow one another) in the order of their range shell,
+ * LES level and x, restored by a counting sort after every `steps` calls of rsc_advance_time (and after an upload of positions); 0
  * keeps the caller's order.  The order is invisible at the ABI: upload and
  * download map the caller's indices, and no result depends on it beyond the
  * rounding of the gate sums.  Default 128. */
@@ -351,10 +351,9 @@ int rsc_rand_sequence(uint32_t seed, uint32_t count, int32_t *out);
  * counts the drops per bin as H->dsd_pop does. */
 int rsc_populate_host(const rsc_populate_args *a, size_t num_scats, float *pos4, float *vel4, float *ori4,
                       float *tum4, float *aux4, float *rcs4, uint32_t *rnd4, uint32_t *dsd_pop);
-/* The same state made straight into an allocated worker: generated on the
- * host in blocks that go to the device by page-locked asynchronous copies
- * while the next block is generated (RS_populate + RS_upload without the
- * full host arrays). */
+/* The same state, bit for bit, made straight into an allocated worker: drawn
+ * on the device from rand()'s states at the start of each chunk of scatterers
+ * (RS_populate + RS_upload without the host arrays). */
 int rsc_populate_upload(rsc_worker *w, const rsc_populate_args *a, uint32_t *dsd_pop);
 const char *rsc_populate_last_error(void);
 

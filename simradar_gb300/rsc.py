@@ -354,7 +354,7 @@ class Worker:
         return s.value or 0
 
     def set_sort_interval(self, steps):
-        """Steps between re-sorts of the background range into spatial
+        """Steps between re-sorts of the scatterers into spatial
         order (0: keep the caller's order)."""
         _check(self._lib.rsc_set_sort_interval(self._h, int(steps)))
 
