@@ -2329,12 +2329,12 @@ int batch_capture(rsc_batch *b, int steps) {
 /* The pos / rcs pairs of every step: step k of a run reads the instance's
  * current pair when k is even, its other pair when k is odd, and the advance
  * writes the other one. */
-void batch_fill_pairs(rsc_batch *b, int steps) {
+void batch_fill_pairs(rsc_batch *b, rsc::BatchStep *row, int steps) {
     const size_t n = b->w.size();
     for (int k = 0; k < steps; k++) {
         for (size_t i = 0; i < n; i++) {
             rsc_worker *x = b->w[i];
-            rsc::BatchStep &S = b->h_steps[(size_t)k * n + i];
+            rsc::BatchStep &S = row[(size_t)k * n + i];
             const bool odd = (k & 1) != 0;
             S.pos_r = odd ? x->pos_next : x->pos;
             S.rcs_r = odd ? x->rcs_next : x->rcs;
@@ -2753,7 +2753,7 @@ int rsc_batch_autotune(rsc_batch *b, const float *sim_descs) {
     s = batch_join_workers(b);
     if (s) return s;
     const size_t n = b->w.size();
-    batch_fill_pairs(b, 1);
+    batch_fill_pairs(b, b->h_steps, 1);
     RSC_CUDA(cudaMemcpyAsync(b->d_steps, b->h_steps, n * sizeof(rsc::BatchStep), cudaMemcpyHostToDevice, b->stream));
     RSC_CUDA(cudaEventRecord(b->ev_h2d, b->stream));
     EventPair ev;
@@ -2966,51 +2966,47 @@ int batch_persist_launch(rsc_batch *b, int steps) {
     return RSC_OK;
 }
 
-int batch_run(rsc_batch *b, int steps, const float *sim_descs, const int *les_ids, float *pulses_out, int use_graph,
-              bool wait) {
-    int s = check_batch(b);
-    if (s) return s;
-    if (steps < 1) return fail(RSC_ERR_ARG, "steps %d", steps);
-    if (sim_descs == nullptr || les_ids == nullptr) return fail(RSC_ERR_ARG, "sim_descs / les_ids is NULL");
-    s = batch_reserve(b, steps);
-    if (s) return s;
-    s = batch_fill_steps(b, steps, sim_descs, les_ids);
-    if (s) return s;
+/* Steps that a run of `steps` takes between sorts of its instances: about equal
+ * parts of at most kNodeBatchSteps or the shortest interval that a worker asked
+ * for, whichever is more (one graph serves all but a shorter last part); the
+ * whole run when a worker keeps the caller's order.  64 instances, runs of 500
+ * steps: 17,141 pulses/s sorted between runs only, 18,638 this way. */
+int batch_part(rsc_batch *b, int steps) {
+    uint64_t most = UINT64_MAX;
     for (rsc_worker *x : b->w) {
-        s = flush_pending(x);
-        if (s) return s;
+        if (x->sort_interval <= 0) return steps;
+        most = std::min(most, (uint64_t)x->sort_interval);
     }
-    s = batch_join_workers(b);
-    if (s) return s;
+    most = std::max(most, (uint64_t)kNodeBatchSteps);
+    const uint64_t parts = ((uint64_t)steps + most - 1) / most;
+    return (int)(((uint64_t)steps + parts - 1) / parts);
+}
+
+/* Steps [k0, k0 + steps) of a run: the sort when it is due, the descriptors,
+ * the launches and the copy of their pulses.  The device's tables and pulses
+ * are the same for every part, in stream order; the host's rows are not. */
+int batch_run_part(rsc_batch *b, int k0, int steps, bool use_graph, float *pulses_out) {
     const size_t n = b->w.size();
+    rsc::BatchStep *row = b->h_steps + (size_t)k0 * n;
+    int s = RSC_OK;
     for (size_t i = 0; i < n; i++) {
-        s = maybe_sort(b->w[i], &b->pops[i], b->h_steps[i].sim, b->stream);
+        rsc_worker *x = b->w[i];
+        if (k0 > 0 && x->sort_interval > 0) {
+            x->sort_due = true;
+            x->sig_aux_stale = false;   /* of a pulse that later ones of this run replace */
+        }
+        s = maybe_sort(x, &b->pops[i], row[i].sim, b->stream);
         if (s) return s;
         /* the advances write both pairs: scatterers outside the population
          * ranges carry over into the other one */
-        s = copy_unadvanced(b->w[i], &b->pops[i], b->stream);
+        s = copy_unadvanced(x, &b->pops[i], b->stream);
         if (s) return s;
     }
-    s = batch_prepare(b, b->h_steps, steps);
+    s = batch_prepare(b, row, steps);
     if (s) return s;
-    batch_fill_pairs(b, steps);
-    /* LES slots this run reads: wait for their pending refills */
-    std::vector<char> used(2 * n, 0);
-    for (size_t r = 0; r < (size_t)steps * n; r++) used[2 * (r % n) + (b->h_steps[r].les_id & 1)] = 1;
-    for (size_t q = 0; q < 2 * n; q++) {
-        if (used[q] && b->slot_pending[q]) {
-            RSC_CUDA(cudaStreamWaitEvent(b->stream, b->slot_ready[q], 0));
-            b->slot_pending[q] = 0;
-        }
-        rsc_worker *x = b->w[q / 2];
-        if (used[q] && x->les_wait[q & 1]) {
-            /* a frame from rsc_les_upload_async */
-            RSC_CUDA(cudaStreamWaitEvent(b->stream, x->les_ready[q & 1], 0));
-            x->les_wait[q & 1] = false;
-        }
-    }
-    RSC_CUDA(cudaMemcpyAsync(b->d_steps, b->h_steps, (size_t)steps * n * sizeof(rsc::BatchStep),
-                             cudaMemcpyHostToDevice, b->stream));
+    batch_fill_pairs(b, row, steps);
+    RSC_CUDA(cudaMemcpyAsync(b->d_steps, row, (size_t)steps * n * sizeof(rsc::BatchStep), cudaMemcpyHostToDevice,
+                             b->stream));
     RSC_CUDA(cudaEventRecord(b->ev_h2d, b->stream));
     if (b->persist && b->mode != RSC_PULSE_F64) {
         s = batch_persist_prepare(b, steps);
@@ -3028,17 +3024,54 @@ int batch_run(rsc_batch *b, int steps, const float *sim_descs, const int *les_id
         b->launches += (uint64_t)steps * (1u + (b->rain_blocks ? 1u : 0u) + (b->deb_blocks ? 1u : 0u));
     }
     batch_swap_pairs(b, steps);
-    for (size_t q = 0; q < 2 * n; q++) {
-        if (used[q]) RSC_CUDA(cudaEventRecord(b->slot_used[q], b->stream));
-    }
+    for (rsc_worker *x : b->w) x->since_sort += (uint64_t)steps;
     if (pulses_out) {
-        RSC_CUDA(cudaMemcpyAsync(pulses_out, b->d_out, (size_t)steps * n * b->Gmax * sizeof(float4),
-                                 cudaMemcpyDeviceToHost, b->stream));
+        RSC_CUDA(cudaMemcpyAsync(pulses_out + (size_t)k0 * n * b->Gmax * 4, b->d_out,
+                                 (size_t)steps * n * b->Gmax * sizeof(float4), cudaMemcpyDeviceToHost, b->stream));
+    }
+    return RSC_OK;
+}
+
+int batch_run(rsc_batch *b, int steps, const float *sim_descs, const int *les_ids, float *pulses_out, int use_graph,
+              bool wait) {
+    int s = check_batch(b);
+    if (s) return s;
+    if (steps < 1) return fail(RSC_ERR_ARG, "steps %d", steps);
+    if (sim_descs == nullptr || les_ids == nullptr) return fail(RSC_ERR_ARG, "sim_descs / les_ids is NULL");
+    s = batch_reserve(b, steps);
+    if (s) return s;
+    s = batch_fill_steps(b, steps, sim_descs, les_ids);
+    if (s) return s;
+    for (rsc_worker *x : b->w) {
+        s = flush_pending(x);
+        if (s) return s;
+    }
+    s = batch_join_workers(b);
+    if (s) return s;
+    const size_t n = b->w.size();
+    /* LES slots this run reads: wait for their pending refills */
+    std::vector<char> used(2 * n, 0);
+    for (size_t r = 0; r < (size_t)steps * n; r++) used[2 * (r % n) + (b->h_steps[r].les_id & 1)] = 1;
+    for (size_t q = 0; q < 2 * n; q++) {
+        if (used[q] && b->slot_pending[q]) RSC_CUDA(cudaStreamWaitEvent(b->stream, b->slot_ready[q], 0));
+        /* a frame from rsc_les_upload_async */
+        rsc_worker *x = b->w[q / 2];
+        if (used[q] && x->les_wait[q & 1]) RSC_CUDA(cudaStreamWaitEvent(b->stream, x->les_ready[q & 1], 0));
+    }
+    const int part = batch_part(b, steps);
+    for (int k0 = 0; k0 < steps; k0 += part) {
+        s = batch_run_part(b, k0, std::min(part, steps - k0), use_graph != 0 && steps - k0 >= part, pulses_out);
+        if (s) return s;
+    }
+    for (size_t q = 0; q < 2 * n; q++) {
+        if (!used[q]) continue;
+        b->slot_pending[q] = 0;
+        b->w[q / 2]->les_wait[q & 1] = false;
+        RSC_CUDA(cudaEventRecord(b->slot_used[q], b->stream));
     }
     RSC_CUDA(cudaEventRecord(b->ev_done, b->stream));
     for (size_t i = 0; i < n; i++) {
         rsc_worker *x = b->w[i];
-        x->since_sort += (uint64_t)steps;
         RSC_CUDA(cudaStreamWaitEvent(x->stream, b->ev_done, 0));
         s = release_main(x);   /* the batch changed the state in place */
         if (s) return s;

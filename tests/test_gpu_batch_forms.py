@@ -68,3 +68,42 @@ def test_advance_forms_match_oracle(backend, oracle_lib, pair, uniform, threads)
     finally:
         for S in pair:
             S.les_desc = stretched
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("form", ["graph", "stream", "persistent", "unsorted"])
+def test_long_run_equals_short_ones(backend, pair, form, precision):
+    """A run long enough to be sorted on its way (300 steps: three parts of
+    100) against the same steps as runs of 77 and 69: states bit for bit, each
+    pulse within the two sums' order (2e-5 of the sums of |w x| a side; those are at most
+    3 times the pulse's largest value here, so 1.2e-4 of that)."""
+    results = []
+    for cuts in ([300], [77, 77, 77, 69]):
+        ws = []
+        for S in pair:
+            W = backend.Worker(0)
+            synth.load_worker(W, S)
+            W.set_precision(precision)
+            if form == "unsorted":
+                W.set_sort_interval(0)
+            ws.append(W)
+        Bt = backend.Batch(ws)
+        Bt.set_populations([synth.population(S) for S in pair])
+        Bt.set_precision(precision)
+        Bt.set_persistent(form == "persistent")
+        pulses, k = [], 0
+        for c in cuts:
+            sims = np.stack([[synth.pulse_sim_desc(S, (k + j) % 60 + i, tic=(k + j) * 1e-3) for i, S in enumerate(pair)]
+                             for j in range(c)]).astype(np.float32)
+            les = np.array([[((k + j) // 50) & 1] * 2 for j in range(c)], np.int32)
+            pulses.append(np.array(Bt.run(sims, les, use_graph=form != "stream")))
+            k += c
+        results.append((np.concatenate(pulses), [W.download(STATE_FIELDS + ("aux", "sig")) for W in ws]))
+        Bt.close()
+        for W in ws:
+            W.close()
+    (pa, sa), (pb, sb) = results
+    for a, b in zip(sa, sb):
+        assert_state_equal(a, b, fields=STATE_FIELDS + ("aux", "sig"))
+    scale = np.abs(pb).max(axis=(2, 3), keepdims=True)
+    assert (scale > 0).all() and (np.abs(pa - pb) <= 1.2e-4 * scale).all()
