@@ -279,6 +279,8 @@ int rsc_batch_get_advance_shape(rsc_batch *b, int *threads, int *blocks_per_sm);
  * float4 per instance, no gain applied) are copied to pulses_out as
  * [k][i][max_gates] float4 if it is not NULL.  With use_graph the 2 * steps
  * launches are captured once in a CUDA graph (per step count) and replayed.
+ * A long run goes in equal parts of at most half the sort interval (64 steps
+ * or more), each instance sorted before each; states do not depend on it.
  * Returns after the pulses are on the host (or the work is queued when
  * pulses_out is NULL; rsc_batch_synchronize waits). */
 int rsc_batch_run(rsc_batch *b, int steps, const float *sim_descs, const int *les_ids, float *pulses_out,

@@ -73,8 +73,9 @@ def test_advance_forms_match_oracle(backend, oracle_lib, pair, uniform, threads)
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("form", ["graph", "stream", "persistent", "unsorted"])
 def test_long_run_equals_short_ones(backend, pair, form, precision):
-    """A run long enough to be sorted on its way (300 steps: three parts of
-    100) against the same steps as runs of 77 and 69: states bit for bit, each
+    """A run long enough to be sorted on its way (300 steps: five parts of 60)
+    against the same steps as runs of 77 and 69 (parts and a shorter last
+    one): states bit for bit, each
     pulse within the two sums' order (2e-5 of the sums of |w x| a side; those are at most
     3 times the pulse's largest value here, so 1.2e-4 of that)."""
     results = []
