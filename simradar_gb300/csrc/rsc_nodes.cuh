@@ -349,16 +349,21 @@ __device__ __noinline__ void comp_stray(const PulseArgs &P, int j, const CompSig
     comp_node(P, j, c, d);
     two_sum(g.r, -c, uh, ul);
     ul = ul + (g.rl - d);
-    /* the quotient can be one off beside a node */
-    const float u = uh + ul;
-    if (u < 0.0f || u >= delta) {
-        const float by = u < 0.0f ? delta : -delta;
-        j += u < 0.0f ? -1 : 1;
-        two_sum(uh, by, a, b);
-        uh = a;
+    /* The quotient can be one off beside a node.  Which side is decided on the
+     * double-float less the node's offset, not on the rounded uh + ul, which is
+     * delta up to half an ulp below it: the next interval's offset would be
+     * negative there and the scatterer in neither. */
+    two_sum(uh, -delta, a, b);
+    if (uh + ul < 0.0f) {
+        j--;
+        two_sum(uh, delta, uh, b);
         ul = ul + b;
+    } else if (a + (b + ul) >= 0.0f) {
+        j++;
+        uh = a;
+        ul = b + ul;
     }
-    if (j < 0 || j > last || !(uh + ul >= 0.0f && uh + ul <= delta)) return;
+    if (j < 0 || j > last) return;
     double *o = P.acc64 + kCompSums * (unsigned)j;
 #pragma unroll 1
     for (int l = 0; l < 4; l++) {

@@ -1,0 +1,79 @@
+"""The compensated pulse where its interval sums are delicate, against the FP64
+pulse of the same state: scatterers within a rounding of a node of the gate
+grid, gates fine beside the range's own spacing, and values near the end of
+FP32's range.
+"""
+import numpy as np
+import pytest
+
+from simradar_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def still_worker(backend, S, one_warp=False):
+    """A worker whose state has been sorted by a step of no length: positions
+    are the scene's, in spatial order."""
+    S.concept = 0
+    S.sim_desc[5] = synth.fbits(0)
+    W = backend.Worker(0)
+    synth.load_worker(W, S)
+    W.set_precision(1)
+    if one_warp:
+        W.set_pulse_shape(1, 1)
+    sd = synth.pulse_sim_desc(S, 50)
+    sd[11] = 0.0
+    W.advance_time(synth.population(S), 0, sd)
+    assert W.sort_count == 1
+    assert np.array_equal(W.download(("pos",))["pos"], S.state["pos"])
+    return W, sd
+
+
+def both(W, sd):
+    W.make_pulse(sd)
+    comp = W.download_pulse(1.0).astype(np.float64)
+    W.set_precision(2)
+    W.make_pulse(sd)
+    ref = W.download_pulse(1.0).astype(np.float64)
+    W.set_precision(1)
+    return comp, ref
+
+
+@pytest.mark.parametrize("start,spacing,node", [
+    (1850.1, 7.5, 27),         # a start FP32 does not hold on the ranges' grid
+    (1850.0, 30.0 / 7.0, 39),  # a spacing it does not hold
+    (1850.0, 15.0, 12),        # both held
+])
+def test_scatterers_just_below_a_node(backend, start, spacing, node):
+    """Scatterers 1e-8 to 6e-7 m below the node that ends a warp's window of two
+    intervals: their offset from its start is the spacing in FP32, yet they
+    belong to it.  The rest of the scatterers, without backscatter, bring the
+    windows there; the pulse is that of the few.
+
+    Tolerance: that of the documented form, 1e-5 of a gate, taken of the
+    largest; a scatterer left out is 1 / sqrt(count) of it."""
+    n, rng = 40000, np.random.default_rng(3)
+    S = synth.make_scene(num_rain=n, gates=int(570 / spacing), gate_spacing=spacing, range_start=start, les_count=1, seed=5)
+    R = float(np.float32(start)) + node * float(np.float32(spacing))
+    few = rng.choice(np.arange(n // 2, n), 1500, replace=False)
+    x0 = rng.uniform(15.0, 25.0, n)
+    r = np.empty(n)
+    r[:n // 2] = R - spacing - rng.uniform(0.01, 0.3, n // 2)
+    r[n // 2:] = R - rng.uniform(0.01, 0.3, n - n // 2)   # one shell of the order
+    r[few] = R - rng.uniform(1e-8, 6e-7, len(few))
+    pos = S.state["pos"]
+    pos[:, 2] = 1.0
+    pos[:, 1] = np.sqrt(r ** 2 - x0 ** 2 - 1.0)
+    y = pos[:, 1].astype(np.float64)
+    pos[:, 0] = np.sqrt(r ** 2 - y ** 2 - 1.0)          # the range to 2e-8 m
+    assert np.isfinite(pos).all()
+    W, sd = still_worker(backend, S, one_warp=True)
+    sd[0], sd[1], sd[2] = synth.beam_unit(0.5, 0.0)
+    rcs = np.zeros((n, 4), np.float32)
+    rcs[few] = rng.standard_normal((len(few), 4))
+    W.upload(0, rcs=rcs)
+    comp, ref = both(W, sd)
+    top = np.abs(ref).max()
+    assert top > 0.0
+    assert (np.abs(comp - ref) <= 1.0e-5 * top).all(), np.abs(comp - ref).max() / top
+    W.close()
