@@ -212,8 +212,9 @@ struct NodeWindow {
  * interval reduced across the warp for every run of 64 with signal_comp's
  * terms; 8.4 M scatterers at 30 km 266 -> 202 us; 77,777 on gates 7.5 m apart
  * (too many for the gate window: every gate visited) 119 -> 15 us.  A gate's
- * error against FP64 is what it was (rms 8.4e-9 of the sum of |x| on a
- * 21,536-scatterer scene, both forms: the output's rounding). */
+ * error against FP64 is what it was or less (rms 8.4e-9 of the sum of |x| on a
+ * 21,536-scatterer scene, both forms: the output's rounding; 1,000 pulses of
+ * 8.4 M at 30 km 2.3e-8 of the gate, 2.7e-8 before). */
 
 /* Add the double-float (h, l) to the double-float sum (S, s). */
 __device__ __forceinline__ void df_acc(float &S, float &s, float h, float l) {

@@ -459,10 +459,12 @@ struct CompSig {
 /* sine and cosine of rh + rl + q pi/2 (|rh| <= 0.8, |rl| <= ulp(rh)) as
  * double-floats, by their Taylor series: the terms r, r^3/6, r^5/120,
  * 1 - r^2/2 and r^4/24 as double-floats, the rest (below 4e-4) in FP32, rl to
- * first order.  Within 1e-10, rms 1e-11: the range's own 2^-48 leaves the
- * phase 3e-10 rad (rms) at 2 km and 5e-9 at 30 km, which the 1e-14 of
- * sincos_df's node table, at twice the operations, cannot better.  qbits: q
- * in its low bits. */
+ * first order.  Within 1.4e-10, rms 2e-11: the range's own 2^-48 leaves the
+ * phase 3e-10 rad (rms) at 2 km and 4e-9 at 30 km, which the 1e-14 of
+ * sincos_df's node table, at twice the operations, cannot better (a term of
+ * signal_comp_mid against FP64, of its |x| W / r^2: rms 8.0e-10 at 1,850 m and
+ * 5.7e-9 at 31,850 m; of signal_comp 2.8e-9 and 6.8e-9).  qbits: q in its low
+ * bits. */
 __device__ __forceinline__ void sincos_series_df(float rh, float rl, unsigned qbits, float &sh, float &sl, float &ch,
                                                  float &cl) {
     float p, pe;
@@ -491,12 +493,17 @@ __device__ __forceinline__ void sincos_series_df(float rh, float rl, unsigned qb
     fast_two_sum(c0, c4, c1, c1e);
     const float s1 = (se + s2e) + (fmaf(t5 * p, ps, c3l + c5l) + rl * c1);
     const float c2 = (ce + c1e) + (fmaf(p2 * p, pc, c4l) - fmaf(0.5f, pe, rl * s0));
+    /* the head takes in its tail: the terms above reach 3e-4 of it, which the
+     * products of a term's tail and a range's would drop (df_mul_pair) */
+    float fsh, fsl, fch, fcl;
+    fast_two_sum(s0, s1, fsh, fsl);
+    fast_two_sum(c1, c2, fch, fcl);
     const bool swap = (qbits & 1u) != 0u;
     const unsigned fs = (qbits & 2u) << 30, fc = ((qbits + 1u) & 2u) << 30;
-    sh = __uint_as_float(__float_as_uint(swap ? c1 : s0) ^ fs);
-    sl = __uint_as_float(__float_as_uint(swap ? c2 : s1) ^ fs);
-    ch = __uint_as_float(__float_as_uint(swap ? s0 : c1) ^ fc);
-    cl = __uint_as_float(__float_as_uint(swap ? s1 : c2) ^ fc);
+    sh = __uint_as_float(__float_as_uint(swap ? fch : fsh) ^ fs);
+    sl = __uint_as_float(__float_as_uint(swap ? fcl : fsl) ^ fs);
+    ch = __uint_as_float(__float_as_uint(swap ? fsh : fch) ^ fc);
+    cl = __uint_as_float(__float_as_uint(swap ? fsl : fcl) ^ fc);
 }
 
 /* signal_comp for scatterers ahead of the beam whose antenna weight lies

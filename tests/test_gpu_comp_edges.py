@@ -77,3 +77,28 @@ def test_scatterers_just_below_a_node(backend, start, spacing, node):
     assert top > 0.0
     assert (np.abs(comp - ref) <= 1.0e-5 * top).all(), np.abs(comp - ref).max() / top
     W.close()
+
+
+def test_gates_fine_beside_the_range(backend):
+    """Gates 1/16 m apart at 31,850 m, where FP32 ranges are 1/512 m apart: the
+    tail of a scatterer's offset in its interval is then a hundredth of the
+    gate, and what a term's tail times it leaves out shows in the gate.
+
+    Tolerance: FP32 output, 2^-24 of the gate, and the range's 2^-48 (1.1e-10 m:
+    1.4e-8 rad of phase, 2e-9 of the gate) added at random; 2^-23 of the
+    largest gate covers both."""
+    n, rng = 4096, np.random.default_rng(4)
+    S = synth.make_scene(num_rain=n, gates=64, gate_spacing=0.0625, range_offset=30000.0, les_count=1, seed=5,
+                         tau=0.125 / 1.5e8)
+    r = rng.uniform(31849.9, 31854.1, n)
+    x, z = rng.uniform(-200.0, 200.0, n), rng.uniform(1.0, 300.0, n)
+    pos = S.state["pos"]
+    pos[:, 0], pos[:, 2] = x, z
+    pos[:, 1] = np.sqrt(r ** 2 - pos[:, 0].astype(np.float64) ** 2 - pos[:, 2].astype(np.float64) ** 2)
+    W, sd = still_worker(backend, S)
+    sd[0], sd[1], sd[2] = synth.beam_unit(0.0, 0.25)
+    W.upload(0, rcs=rng.standard_normal((n, 4)).astype(np.float32))
+    comp, ref = both(W, sd)
+    top = np.abs(ref).max()
+    assert (np.abs(comp - ref) <= 2.0 ** -23 * top).all(), np.abs(comp - ref).max() / top
+    W.close()
