@@ -311,8 +311,9 @@ int rsc_batch_set_les_async(rsc_batch *b, int index, int slot, const float *uvwt
  * and advances them; no block waits for another (the pulses of different
  * steps use separate accumulators, the last block of an instance's pulse
  * converting it).  The state and the pulses are the ones of the three-launch
- * form.  The FP64 precision mode always runs the three-launch form; use_graph
- * is ignored while this is on. */
+ * form.  The FP64 precision mode, and a batch with an instance whose range
+ * weight reaches more than seven gates, always run the three-launch form;
+ * use_graph is ignored otherwise while this is on. */
 int rsc_batch_set_persistent(rsc_batch *b, int enable);
 /* The largest gate count of the batch (the row length of pulses_out). */
 int rsc_batch_max_gates(rsc_batch *b, int *max_gates);

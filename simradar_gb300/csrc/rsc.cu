@@ -1982,6 +1982,7 @@ struct rsc_batch {
     int rain_form = 0;           /* what its kernel is compiled for: rain_kernel */
     bool nodes = false; /* the pulse through the node sums */
     bool tri = false;   /* the pulse kernel with the triangle range weight compiled in */
+    bool persist_now = false; /* the next run in the persistent form */
     /* per-instance launch descriptors and block prefixes */
     std::vector<rsc::BatchAdvance> h_adv;
     std::vector<PulseArgs> h_pulse;
@@ -2081,6 +2082,7 @@ int batch_prepare(rsc_batch *b, const rsc::BatchStep *row, int steps) {
     b->h_deb_prefix.assign(n + 1, 0u);
     b->h_pulse_prefix.assign(n + 1, 0u);
     bool tri = true;   /* every instance's range table is the triangle */
+    bool window = true;   /* every instance's range weight fits the gate window */
     b->concept.assign(n, 0u);
     unsigned acc_r = 0, acc_d = 0, acc_p = 0;
     bool nodes = true;
@@ -2121,14 +2123,17 @@ int batch_prepare(rsc_batch *b, const rsc::BatchStep *row, int steps) {
             P.runs = x->runs;
         }
         P.materialize = 0;
-        if (b->mode != RSC_PULSE_F64 && !b->persist && steps <= kNodeBatchSteps) use_nodes(x, P, b->mode, true);
+        if (b->mode != RSC_PULSE_F64 && steps <= kNodeBatchSteps) use_nodes(x, P, b->mode, true);
         nodes = nodes && P.mom_n > 0;
         max_n = std::max(max_n, P.mom_n);
         tri = tri && P.rw_tri;
+        window = window && !P.dense;
         b->concept[i] = rsm_f2u(row[i].sim[5]);
     }
+    /* the persistent form sums in the gate window */
+    b->persist_now = b->persist && b->mode != RSC_PULSE_F64 && window;
     /* through the node sums when every instance's pulse may */
-    nodes = nodes && b->mode != RSC_PULSE_F64 && !b->persist;
+    nodes = nodes && b->mode != RSC_PULSE_F64 && !b->persist_now;
     if (!nodes) {
         /* the sums gate by gate, or their moments per interval */
         for (size_t i = 0; i < n; i++) {
@@ -3010,7 +3015,7 @@ int batch_run_part(rsc_batch *b, int k0, int steps, bool use_graph, float *pulse
     RSC_CUDA(cudaMemcpyAsync(b->d_steps, row, (size_t)steps * n * sizeof(rsc::BatchStep), cudaMemcpyHostToDevice,
                              b->stream));
     RSC_CUDA(cudaEventRecord(b->ev_h2d, b->stream));
-    if (b->persist && b->mode != RSC_PULSE_F64) {
+    if (b->persist_now) {
         s = batch_persist_prepare(b, steps);
         if (s == RSC_OK) s = batch_persist_launch(b, steps);
         if (s) return s;

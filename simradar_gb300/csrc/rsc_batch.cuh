@@ -197,8 +197,9 @@ k_pulse_batch(const PulseArgs *inst, const BatchStep *steps, const unsigned *pre
     const int i = batch_pulse_args(sp, s_i, inst, steps, prefix, ninst, out, out_stride);
     const unsigned b0 = __ldg(prefix + i);
     /* an instance whose state is in spatial order takes two scatterers per
-     * lane, as the one-instance kernel does */
-    if (MODE != 2 && sp.coherent_span > 0 && !sp.materialize) {
+     * lane, as the one-instance kernel does; a range weight too wide for the
+     * gate window visits every gate */
+    if (MODE != 2 && sp.coherent_span > 0 && !sp.materialize && !sp.dense) {
         pulse_body_group<MODE == 2 ? 0 : MODE, 2, TRI>(sp, blockIdx.x - b0, __ldg(prefix + i + 1) - b0);
     } else {
         pulse_body<MODE>(sp, blockIdx.x - b0, __ldg(prefix + i + 1) - b0);
