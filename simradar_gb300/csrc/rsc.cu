@@ -94,6 +94,9 @@ struct rsc_worker {
     float *rk = nullptr, *rk_hi = nullptr, *rk_lo = nullptr;
     double *rk64 = nullptr;
     float *node = nullptr;        /* node positions -kNodeMaxN .. G - 1 + kNodeMaxN (rsc_nodes.cuh) */
+    double slip = 0.0;            /* node_slip of these gates for the triangle below (slip_n 0: not known) */
+    int slip_n = 0;
+    float slip_scale = 0.0f;
     double *acc64 = nullptr;      /* the pulse kernel's FP64 grid accumulator */
     unsigned *counter = nullptr;
     unsigned long long *runs = nullptr;   /* the compensated pulse's run counter */
@@ -434,6 +437,7 @@ int set_gates(rsc_worker *w) {
     RSC_CUDA(cudaMemcpy(w->rk_lo, lo.data(), G * sizeof(float), cudaMemcpyHostToDevice));
     RSC_CUDA(cudaMemcpy(w->rk64, r64.data(), G * sizeof(double), cudaMemcpyHostToDevice));
     /* the nodes: the running sum's origins, continued evenly on both sides */
+    w->slip_n = 0;
     std::vector<float> nd(rsc::node_count(G, rsc::kNodeMaxN));
     for (int m = -rsc::kNodeMaxN; m < (int)G + rsc::kNodeMaxN; m++) {
         const int k = std::min(std::max(m, 0), (int)G - 1);
@@ -666,6 +670,36 @@ int node_span(const PulseArgs &P) {
     return (int)n;
 }
 
+/* The weight by which the triangle of half width 1 / scale (n gate spacings)
+ * misses the nodes at its ends: the nodes are the FP32 running sum of the gate
+ * origins, whose steps differ from the spacing where FP32 does not hold it (30 m
+ * / 9: 2.4e-5 at 1,850 m; 30 m / 11: 2.6e-4 at 31,850 m; 0.6 m, 512 gates:
+ * 9.6e-3 at 60 km), and every scatterer of an end's interval would have that
+ * weight too much or too little. */
+double node_slip(float start, float delta, uint32_t G, int n, float scale) {
+    std::vector<float> rk(G);
+    float r = start;
+    for (uint32_t k = 0; k < G; k++) {
+        rk[k] = r;
+        r = r + delta;
+    }
+    const auto node = [&](int m) {   /* as set_gates */
+        const int k = std::min(std::max(m, 0), (int)G - 1);
+        return (double)(float)((double)rk[k] + (double)(m - k) * (double)delta);
+    };
+    double slip = 0.0;
+    for (int k = 0; k < (int)G; k++) {
+        slip = std::max(slip, fabs((node(k + n) - (double)rk[k]) * (double)scale - 1.0));
+        slip = std::max(slip, fabs(((double)rk[k] - node(k - n)) * (double)scale - 1.0));
+    }
+    return slip;
+}
+
+/* ... up to which the plain sums go through the nodes: what pass 1 itself
+ * rounds off a weight (its product and its sum, 2^-24 each).  Spacings that
+ * FP32 holds at the range are within 2^-24, the rounding of the scale. */
+constexpr double kNodeSlip = 0x1p-23;
+
 /* The margin, in gates, by which the sparse path widens the exact support
  * d_lo .. d_hi (metres) of the range weight: the measured drift of the FP32
  * running-sum gate origins from exact spacing; two ulps of the largest range
@@ -694,7 +728,8 @@ constexpr int kNodeBatchSteps = 128;
  * 77 gates 7.5 m apart 1875 us), the other grows with the gates (1670). */
 constexpr uint32_t kStrayGates = 82;
 
-/* A pulse through the node sums where the triangle allows them.
+/* A pulse through the node sums where the triangle allows them; the plain one
+ * only where the triangle's ends meet the nodes (node_slip).
  * On a state in spatial order always, unless rsc_set_pulse_moments turned the
  * compensated ones off.  Out of it (before the first sort, after an upload)
  * plain scatterer by scatterer when the triangle is wide enough for that
@@ -706,6 +741,14 @@ constexpr uint32_t kStrayGates = 82;
 void use_nodes(rsc_worker *w, PulseArgs &P, int mode, bool batch) {
     const int n = node_span(P);
     if (n == 0 || (mode != RSC_PULSE_PLAIN && !w->moments)) return;
+    if (mode == RSC_PULSE_PLAIN) {
+        if (w->slip_n != n || w->slip_scale != P.rwd[0]) {
+            w->slip = node_slip(w->range_start, w->range_delta, w->G, n, P.rwd[0]);
+            w->slip_n = n;
+            w->slip_scale = P.rwd[0];
+        }
+        if (w->slip > kNodeSlip) return;   /* pass 1's own weights, gate by gate */
+    }
     const bool ordered = w->perm != nullptr && !w->sort_due && w->since_sort < kOrderedSteps;
     if (!ordered && mode == RSC_PULSE_PLAIN) {
         if (!batch && P.coherent_span <= 0 && n >= rsc::kNodeAnyLeast &&
@@ -3367,7 +3410,7 @@ int rsc_make_pulse_noalloc(const float *pos4, const float *rcs4, size_t num_scat
     /* scatterer by scatterer onto the nodes where the triangle allows it: 48 KB
      * hold the sums of any G here, so the launch needs no query */
     setup.n = node_span(P);
-    if (setup.n < rsc::kNodeAnyLeast) setup.n = 0;
+    if (setup.n < rsc::kNodeAnyLeast || node_slip(range_start, range_delta, G, setup.n, P.rwd[0]) > kNodeSlip) setup.n = 0;
     if (setup.n > 0) {
         P.mom_n = setup.n;
         P.any = 1;

@@ -11,7 +11,10 @@
  * and the last block forms every gate from its 2 n - 1 nodes.  The work per
  * scatterer does not depend on n: a pulse sampled finely in range costs what
  * a coarse one does.  The nodes are the gate origins the reference's running
- * sum gives (rs.cl:1214), continued evenly on both sides.
+ * sum gives (rs.cl:1214), continued evenly on both sides.  Where that sum
+ * drifts from the spacing, the triangle's ends miss the nodes and the plain
+ * sums stay gate by gate (node_slip in rsc.cu); the compensated ones use the
+ * even grid and end where the table does.
  *
  * Each warp takes a contiguous piece of the state, 64 neighbours at a time,
  * lane l holding scatterers l and l + 32.  A state in spatial order keeps a
