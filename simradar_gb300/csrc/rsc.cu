@@ -109,7 +109,7 @@ struct rsc_worker {
     float *angular_weight = nullptr;
     uint32_t angular_n = 0;
     float angular_desc[4] = {0};
-    bool angular_finite = true;
+    bool angular_small = true;    /* every weight below 2^20 */
     float4 *ellipsoid = nullptr;
     uint32_t ellipsoid_n = 0;
     float ellipsoid_desc[4] = {0};
@@ -771,11 +771,12 @@ void use_nodes(rsc_worker *w, PulseArgs &P, int mode, bool batch) {
     P.stray = reinterpret_cast<float4 *>(w->acc64 + (2 * rsc::node_count(w->G, rsc::kNodeMaxN) + w->G) * 4);
     P.lead = ordered ? w->sort_end : 0;
     /* half a gate more than the triangles reach; everything when an antenna
-     * weight is not finite, which any range meets */
+     * weight is not finite, which any range meets, or so large that a term may
+     * not be */
     const double lo = (double)w->range_start - (n + 0.5) * (double)w->range_delta;
     const double hi = (double)w->range_start + (w->G - 1 + n + 0.5) * (double)w->range_delta;
-    P.reach_lo2 = lo > 0.0 && w->angular_finite ? (float)(lo * lo) : 0.0f;
-    P.reach_hi2 = hi > 0.0 && w->angular_finite ? (float)(hi * hi) : INFINITY;
+    P.reach_lo2 = lo > 0.0 && w->angular_small ? (float)(lo * lo) : 0.0f;
+    P.reach_hi2 = hi > 0.0 && w->angular_small ? (float)(hi * hi) : INFINITY;
 }
 
 void fill_pulse_args(rsc_worker *w, PulseArgs &P, const float *sim) {
@@ -1030,8 +1031,8 @@ int rsc_set_angular_weight(rsc_worker *w, const float *table, uint32_t n, const 
     s = upload_floats(&w->angular_weight, table, n);
     if (s) return s;
     w->angular_n = n;
-    w->angular_finite = true;
-    for (uint32_t k = 0; k < n; k++) w->angular_finite = w->angular_finite && fabsf(table[k]) < INFINITY;
+    w->angular_small = true;
+    for (uint32_t k = 0; k < n; k++) w->angular_small = w->angular_small && fabsf(table[k]) < 0x1p20f;
     memcpy(w->angular_desc, desc, sizeof(w->angular_desc));
     return RSC_OK;
 }

@@ -688,16 +688,27 @@ __device__ __forceinline__ void node_run(const PulseArgs &P, NodeWindow &W, cons
         node_settle(P, W, g, in, part, bins, stray, lane);
     }
 }
+/* A beam and wave number whose terms are finite for every scatterer that
+ * comp_run may skip: |b| of 2^-20 to 2^20, |k| below 2^12 (a phase below 2^32).
+ * NaN and infinities are neither. */
+__device__ __forceinline__ bool comp_tame(const PulseArgs &P) {
+    const float *sd = P.sim;
+    return fabsf(sd[0]) < 0x1p20f && fabsf(sd[1]) < 0x1p20f && fabsf(sd[2]) < 0x1p20f && fabsf(sd[4]) < 0x1p12f &&
+           P.ib2_hi < 0x1p40f;
+}
+
 __device__ __forceinline__ void comp_run(const PulseArgs &P, CompWindow &W, const float4 *p, const float4 *x, unsigned in,
-                                         int part, unsigned lane) {
+                                         int part, bool tame, unsigned lane) {
     /* nothing to do when no scatterer of the run reaches a gate and none has
-     * a non-finite value, which would reach all of them */
-    bool live = false;
+     * a term that is not finite, which would reach all of them: backscatter
+     * below 2^30 (2^98 times it is finite), ranges of 2^-10 to 2^20 m, and a
+     * pulse that comp_tame */
+    bool live = !tame;
 #pragma unroll
     for (int q = 0; q < 2; q++) {
         const float r2 = fmaf(p[q].x, p[q].x, fmaf(p[q].y, p[q].y, p[q].z * p[q].z));
-        const float f = fmaf(x[q].x, 0.0f, fmaf(x[q].y, 0.0f, fmaf(x[q].z, 0.0f, x[q].w * 0.0f)));
-        live = live || !(f == 0.0f && ((r2 > 0x1p-40f && r2 < P.reach_lo2) || (r2 > P.reach_hi2 && r2 < INFINITY)));
+        const float f = fmaf(x[q].x, 0x1p98f, fmaf(x[q].y, 0x1p98f, fmaf(x[q].z, 0x1p98f, x[q].w * 0x1p98f)));
+        live = live || !(fabsf(f) < INFINITY && ((r2 > 0x1p-20f && r2 < P.reach_lo2) || (r2 > P.reach_hi2 && r2 < 0x1p40f)));
     }
     if (!__any_sync(0xffffffffu, live)) return;
     CompSig g[2];
@@ -759,6 +770,7 @@ __device__ __forceinline__ void node_body(const PulseArgs &P, unsigned blk, unsi
         C.c = -1;
         C.Eh = NAN;
     }
+    const bool tame = MODE == 1 && comp_tame(P);
     const auto next = [&](unsigned long long r) {
         r++;
         return r == last ? lead + me : (r > last ? r + (warps - 1) : r);
@@ -789,7 +801,7 @@ __device__ __forceinline__ void node_body(const PulseArgs &P, unsigned blk, unsi
         if constexpr (MODE == 0) {
             node_run(P, W, p, x, in, part, bins, stray, lane);
         } else {
-            comp_run(P, C, p, x, in, part, lane);
+            comp_run(P, C, p, x, in, part, tame, lane);
         }
     }
     if (MODE == 0) W.flush(bins, lane);

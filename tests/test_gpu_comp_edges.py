@@ -102,3 +102,29 @@ def test_gates_fine_beside_the_range(backend):
     top = np.abs(ref).max()
     assert (np.abs(comp - ref) <= 2.0 ** -23 * top).all(), np.abs(comp - ref).max() / top
     W.close()
+
+
+@pytest.mark.parametrize("word,value", [(0, np.nan), (1, np.inf), (4, np.nan), (4, np.inf)])
+def test_beam_that_is_not_finite(backend, word, value):
+    """A wave number that is not finite makes every scatterer's term NaN, and NaN
+    times a weight of 0 reaches every gate: also when no scatterer is in a
+    gate's reach, as in the FP64 pulse and the sums gate by gate.  (A beam that
+    is not finite leaves the terms finite, on the antenna table's end.)"""
+    n = 1024
+    S = synth.make_scene(num_rain=n, gates=10, les_count=1, seed=5)
+    rng = np.random.default_rng(6)
+    az, el = np.radians(rng.uniform(-7.0, 7.0, n)), np.radians(rng.uniform(1.0, 15.0, n))
+    pos = S.state["pos"]
+    pos[:, 0], pos[:, 1] = 2300.0 * np.cos(el) * np.sin(az), 2300.0 * np.cos(el) * np.cos(az)
+    pos[:, 2] = 2300.0 * np.sin(el)                    # gates up to 2,015 m
+    W, sd = still_worker(backend, S)
+    comp, ref = both(W, sd)
+    assert (comp == 0.0).all() and (ref == 0.0).all()
+    sd[word] = value
+    comp, ref = both(W, sd)
+    W.set_moments(False)
+    gates, _ = both(W, sd)
+    assert np.array_equal(np.isnan(comp), np.isnan(gates))
+    if word == 4:
+        assert np.isnan(ref).all() and np.isnan(comp).all()
+    W.close()
