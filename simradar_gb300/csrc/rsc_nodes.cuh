@@ -252,22 +252,28 @@ __device__ __forceinline__ void comp_node(const PulseArgs &P, int j, float &h, f
     fast_two_sum(s, e + b, h, l);
 }
 
-/* f as a double by its bits: the FP64 units' conversions issue at 1/64 of the
- * FP32 rate.  Values below 2^-126 count as 0. */
+/* f 2^-896 as a double: its exponent as it stands under the wider bias, exact
+ * for subnormal values too.  (The FP64 units' conversions issue at 1/64 of the
+ * FP32 rate: 8.4 M scatterers, 3 steps, 1,025 us with them, 930 without.)  An
+ * infinity or NaN stays one in the head of a double-float, which makes the
+ * sum one whatever the tail gives. */
+constexpr double kWideScale = 0x1p896;
+template <bool HEAD>
 __device__ __forceinline__ double wide_of(float f) {
     const unsigned b = __float_as_uint(f), m = b & 0x7fffffffu;
-    const unsigned hi = (m >> 3) + 0x38000000u, lo = b << 29;
-    return m < 0x00800000u ? 0.0 : __hiloint2double((int)(hi | (b & 0x80000000u)), (int)lo);
+    unsigned hi = (m >> 3) | (b & 0x80000000u);
+    if (HEAD && m >= 0x7f800000u) hi |= 0x7ff00000u;
+    return __hiloint2double((int)hi, (int)(b << 29));
 }
-/* A double-float into a sum in L2, as two reductions: the additions happen
- * there, not in the SM's few FP64 lanes.  (As atomicAdd through a generic
+/* A double-float into a sum in L2 (of 2^-896 times the values), as two
+ * reductions: the additions happen there, not in the SM's few FP64 lanes.  (As atomicAdd through a generic
  * pointer each waited for its answer: 3 us per scatterer.) */
 __device__ __forceinline__ void red_add(double *o, double v) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(o), "d"(v) : "memory");
 }
 __device__ __forceinline__ void red_add_df(double *o, float h, float l) {
-    red_add(o, wide_of(h));
-    red_add(o, wide_of(l));
+    red_add(o, wide_of<true>(h));
+    red_add(o, wide_of<false>(l));
 }
 
 /* The compensated sums of an interval [E_j, E_j+1) between two nodes of the
@@ -275,7 +281,7 @@ __device__ __forceinline__ void red_add_df(double *o, float h, float l) {
  * the last block forms every gate exactly (the triangle's end lies where its
  * table's scale puts it, a few ulps off the node: an interval's own line is
  * right up to there, where node sums would mix it with its neighbour's).
- * Doubles acc64[8 j + l] and acc64[8 j + 4 + l]. */
+ * Doubles acc64[8 j + l] and acc64[8 j + 4 + l], scaled as wide_of. */
 constexpr unsigned kCompSums = 8;
 
 /* A warp's window of two intervals beside the node E, with t = r - E: below
@@ -582,7 +588,7 @@ __device__ __forceinline__ void node_gates(const PulseArgs &P, double *bins, uns
     if constexpr (MODE == 1) {
         const unsigned all = nodes * kCompSums;
 #pragma unroll 4
-        for (unsigned o = threadIdx.x; o < all; o += blockDim.x) bins[o] = __ldcg(P.acc64 + o);
+        for (unsigned o = threadIdx.x; o < all; o += blockDim.x) bins[o] = __ldcg(P.acc64 + o) * kWideScale;
         __syncthreads();
         for (unsigned o = threadIdx.x; o < all; o += blockDim.x) P.acc64[o] = 0.0;
         const double s = (double)P.rwd[0], ds = (double)P.rdelta * s;
@@ -717,7 +723,8 @@ __device__ __forceinline__ void comp_run(const PulseArgs &P, CompWindow &W, cons
 #pragma unroll
     for (int q = 0; q < 2; q++) {
         signal_comp_any(P, p[q], x[q], g[q]);
-        /* NaN or an infinity in any lane makes the sum NaN */
+        /* NaN or an infinity in any lane makes the sum NaN (a tail is finite
+         * where its head is) */
         const float f = fmaf(g[q].s[0], 0.0f, fmaf(g[q].s[1], 0.0f, fmaf(g[q].s[2], 0.0f, g[q].s[3] * 0.0f)));
         W.offset(g[q], th[q], tl[q]);
         const float t = th[q] + tl[q];

@@ -128,3 +128,31 @@ def test_beam_that_is_not_finite(backend, word, value):
     if word == 4:
         assert np.isnan(ref).all() and np.isnan(comp).all()
     W.close()
+
+
+@pytest.mark.parametrize("r,x", [(20.0, 3.0e38), (10.0, 1.0e38), (20.0, 1.0e-33)])
+def test_sums_at_the_ends_of_fp32(backend, r, x):
+    """512 equal terms whose sums, or moments, pass FP32's largest value, and
+    whose tails are below its smallest normal: a gate is the FP64 one, to 1e-5
+    and to 2^-23 of the terms (the triangle's ends are where its FP32 scale
+    puts them, 2^-24 of a weight off the nodes), or not finite where a sum on
+    the way cannot be held, never another finite value."""
+    n = 512
+    S = synth.make_scene(num_rain=n, gates=3, range_start=10.0, les_count=1, seed=5,
+                         box=(-50.0, 1.0, -50.0, 100.0, 100.0, 100.0))
+    pos = S.state["pos"]
+    pos[:, :3] = 0.0, r, 0.0
+    pos[:, 0] = np.linspace(-1e-3, 1e-3, n)
+    W, sd = still_worker(backend, S)
+    sd[0], sd[1], sd[2] = 0.0, 1.0, 0.0
+    W.upload(0, rcs=np.tile(np.array([x, 0.0, x, 0.0], np.float32), (n, 1)))
+    with np.errstate(over="ignore"):
+        comp, ref = both(W, sd)
+    ok = np.isfinite(comp)
+    fits = np.isfinite(ref)
+    lim = 1.0e-5 * np.abs(ref) + 2.0 ** -23 * n * x / r ** 2
+    bad = ok & ~(fits & (np.abs(comp - np.where(fits, ref, 0.0)) <= lim))
+    assert not bad.any(), (comp, ref)
+    if x < 1.0:
+        assert ok.all()
+    W.close()
