@@ -1387,7 +1387,8 @@ static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *si
 
 /* aux / sig of the latest pulse (scat_sig_aux, rs.cl:1050-1110) when the
  * pulse kernel did not write them: formed on `st` from the pos / rcs pair
- * that pulse read and its descriptor.  rs.c's RS_download returns what the
+ * that pulse read and its descriptor, once: a step does not change them.
+ * rs.c's RS_download returns what the
  * last scat_sig_aux launch wrote, so they are formed before anything
  * overwrites or reorders that pair (a second advance, a sort, an upload), or
  * on download.  A batch run's pulses write both for every scatterer, so it
@@ -1761,7 +1762,6 @@ int rsc_advance_time(rsc_worker *w, const rsc_population *pop, int les_id, const
         w->pend_blocks = blocks;
         w->pend_pop = *pop;
         memcpy(w->pend_sim, sim_desc, sizeof(w->pend_sim));
-        w->sig_aux_stale = true;
         return RSC_OK;
     }
     /* on the advance stream, beside the pulse of this step: read the current
@@ -1794,7 +1794,6 @@ int rsc_advance_time(rsc_worker *w, const rsc_population *pop, int les_id, const
     std::swap(w->rcs, w->rcs_next);
     std::swap(w->ev_read, w->ev_read_next);
     std::swap(w->read_pending, w->read_next_pending);
-    w->sig_aux_stale = true;
     w->since_sort++;
     return maybe_sort(w, pop, sim_desc, w->stream);
 }
@@ -1815,6 +1814,11 @@ int rsc_update_debris_rcs(rsc_worker *w, const rsc_population *pop, const float 
     s = fill_debris(w, pop, a, &deb);
     if (s) return s;
     if (deb == 0) return RSC_OK;
+    if (w->sa_rcs == nullptr || w->sa_rcs == w->rcs) {
+        /* the latest pulse's pair is overwritten in place */
+        s = settle_sig_aux(w, w->stream);
+        if (s) return s;
+    }
     unsigned blocks = (unsigned)((deb + rsc::kAdvanceThreads - 1) / rsc::kAdvanceThreads);
     rsc::k_db_rcs<<<blocks, rsc::kAdvanceThreads, 0, w->stream>>>(a);
     RSC_CUDA(cudaGetLastError());
@@ -2531,6 +2535,8 @@ int rsc_autotune(rsc_worker *w, const float sim_desc[16], int *warps_out, int *b
     memcpy(w->last_sim, sim_desc, sizeof(w->last_sim));
     w->have_pulse_desc = true;
     w->sig_aux_stale = true;
+    w->sa_pos = P.pos;
+    w->sa_rcs = P.rcs;
     if (warps_out) *warps_out = best_w;
     if (blocks_per_sm_out) *blocks_per_sm_out = best_p;
     return RSC_OK;
