@@ -200,8 +200,9 @@ int rsc_get_advance_stream(rsc_worker *w, void **stream);
  * types' ranges do not follow one another) in the order of their range shell,
  * LES level and x, restored by a counting sort after every `steps` calls of rsc_advance_time (and after an upload of positions); 0
  * keeps the caller's order.  The order is invisible at the ABI: upload and
- * download map the caller's indices, and no result depends on it beyond the
- * rounding of the gate sums.  Default 128. */
+ * download map the caller's indices, a population whose ranges cut through
+ * those of an earlier one has them back in the caller's order first, and no
+ * result depends on it beyond the rounding of the gate sums.  Default 128. */
 int rsc_set_sort_interval(rsc_worker *w, int steps);
 /* Number of sorts the worker has made. */
 int rsc_sort_count(rsc_worker *w, uint64_t *count);

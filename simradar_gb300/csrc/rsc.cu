@@ -151,6 +151,9 @@ struct rsc_worker {
     int sort_interval = 128;
     uint64_t since_sort = 0;
     uint64_t sort_end = 0;    /* slots [0, sort_end) are in spatial order */
+    /* slots whose scatterers have been reordered among themselves: disjoint,
+     * each the caller's range of the same bounds in another order */
+    std::vector<std::pair<uint64_t, uint64_t>> mixed;
     bool sort_due = true;
     unsigned *perm = nullptr, *perm_alt = nullptr, *inv = nullptr;
     unsigned *sort_key = nullptr, *sort_order = nullptr, *sort_hist = nullptr, *sort_blocks = nullptr;
@@ -259,6 +262,8 @@ void free_sort(rsc_worker *w) {
     }
     w->sort_due = true;
     w->since_sort = 0;
+    w->sort_end = 0;
+    w->mixed.clear();
 }
 
 /* The eight attribute arrays as 16-byte elements, in a fixed order. */
@@ -1245,12 +1250,43 @@ constexpr unsigned kMaxShells = rsc::kMaxSortCells / 32;
 
 static unsigned grid_of(unsigned long long n, unsigned threads) { return (unsigned)((n + threads - 1) / threads); }
 
+/* Slots [origin, origin + count) in the order of w->sort_order (relative to
+ * origin, source of each slot): every attribute array and perm move to the
+ * second buffer set, which then becomes the current one. */
+static int permute_slots(rsc_worker *w, unsigned long long origin, unsigned long long count, cudaStream_t st) {
+    const unsigned long long numel = w->numel;
+    uint4 **arr[8];
+    attribute_arrays(w, arr);
+    rsc::PermuteArgs p;
+    for (int k = 0; k < 8; k++) {
+        p.src[k] = *arr[k];
+        p.dst[k] = w->alt[k];
+    }
+    p.perm_src = w->perm;
+    p.perm_dst = w->perm_alt;
+    p.origin = origin;
+    p.count = count;
+    p.numel = numel;
+    p.order = w->sort_order;
+    rsc::k_sort_permute<<<grid_of(numel, rsc::kSortThreads), rsc::kSortThreads, 0, st>>>(p);
+    for (int k = 0; k < 8; k++) {
+        uint4 *t = *arr[k];
+        *arr[k] = w->alt[k];
+        w->alt[k] = t;
+    }
+    unsigned *t = w->perm;
+    w->perm = w->perm_alt;
+    w->perm_alt = t;
+    rsc::k_sort_inverse<<<grid_of(numel, rsc::kSortThreads), rsc::kSortThreads, 0, st>>>(w->perm, w->inv, numel);
+    RSC_CUDA(cudaGetLastError());
+    w->launches += 2;
+    return RSC_OK;
+}
+
 /* Counting sort of the type ranges into spatial order, each within itself:
  * range shells of a quarter gate, LES levels, x, over the scan box (sim_desc
  * s8-s10 origin, s12-s14 size): rsc_sort.cuh.  Ranges that do not follow one
- * another leave all but the background in the caller's order.  Every
- * attribute array and perm move to the second buffer set, which then becomes
- * the current one. */
+ * another leave all but the background in the caller's order. */
 static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *sim, cudaStream_t st) {
     const unsigned long long origin = pop->origins[0];
     unsigned long long count = pop->counts[0];
@@ -1350,37 +1386,22 @@ static int sort_worker(rsc_worker *w, const rsc_population *pop, const float *si
     rsc::k_scan_add<<<nb, rsc::kScanThreads, 0, st>>>(w->sort_hist, H, w->sort_blocks);
     rsc::k_sort_scatter<<<grid_of(count, rsc::kSortThreads), rsc::kSortThreads, 0, st>>>(w->sort_key, count,
                                                                                         w->sort_hist, w->sort_order);
-    uint4 **arr[8];
-    attribute_arrays(w, arr);
-    rsc::PermuteArgs p;
-    for (int k = 0; k < 8; k++) {
-        p.src[k] = *arr[k];
-        p.dst[k] = w->alt[k];
+    int e = permute_slots(w, origin, count, st);
+    if (e) return e;
+    /* the ranges are mixed now, with what they hold of earlier ones */
+    for (int t = 0; t < a.nranges; t++) {
+        const uint64_t lo = origin + (t ? a.range[t - 1].end : 0), hi = origin + a.range[t].end;
+        auto &m = w->mixed;
+        m.erase(std::remove_if(m.begin(), m.end(), [&](const auto &b) { return b.first >= lo && b.second <= hi; }), m.end());
+        if (hi > lo) m.emplace_back(lo, hi);
     }
-    p.perm_src = w->perm;
-    p.perm_dst = w->perm_alt;
-    p.origin = origin;
-    p.count = count;
-    p.numel = numel;
-    p.order = w->sort_order;
-    rsc::k_sort_permute<<<grid_of(numel, rsc::kSortThreads), rsc::kSortThreads, 0, st>>>(p);
-    for (int k = 0; k < 8; k++) {
-        uint4 *t = *arr[k];
-        *arr[k] = w->alt[k];
-        w->alt[k] = t;
-    }
-    unsigned *t = w->perm;
-    w->perm = w->perm_alt;
-    w->perm_alt = t;
-    rsc::k_sort_inverse<<<grid_of(numel, rsc::kSortThreads), rsc::kSortThreads, 0, st>>>(w->perm, w->inv, numel);
-    RSC_CUDA(cudaGetLastError());
     /* ranges dense enough for a run of 64 to lie in a few shells */
     w->sort_end = 0;
     for (int t = 0; t < a.nranges && origin == 0; t++) {
         if (a.range[t].end - w->sort_end < 8ull * a.shells) break;
         w->sort_end = a.range[t].end;
     }
-    w->launches += 8;
+    w->launches += 6;
     w->sorts++;
     return RSC_OK;
 }
@@ -1408,6 +1429,41 @@ static int settle_sig_aux(rsc_worker *w, cudaStream_t st) {
     w->launches++;
     w->sig_aux_stale = false;
     return RSC_OK;
+}
+
+/* A population whose ranges cut through slots that an earlier one's sort
+ * mixed would act on other scatterers than the caller's: those slots return
+ * to the caller's order first (an order that fits is left alone). */
+static int match_order(rsc_worker *w, const rsc_population *pop, cudaStream_t st) {
+    bool moved = false;
+    for (size_t q = 0; q < w->mixed.size();) {
+        const uint64_t lo = w->mixed[q].first, hi = w->mixed[q].second;
+        bool cut = false;
+        for (int k = 0; k < RSC_MAX_TYPES; k++) {
+            const uint64_t a = pop->origins[k], b = a + pop->counts[k];
+            if (pop->counts[k] != 0 && a < hi && b > lo) cut = cut || a > lo || b < hi;
+        }
+        if (!cut) {
+            q++;
+            continue;
+        }
+        int s = RSC_OK;
+        if (!moved) {
+            /* the arrays move: after the advance stream, before its next advance */
+            s = join_adv(w);
+            if (s == RSC_OK) s = settle_sig_aux(w, st);
+            if (s) return s;
+        }
+        rsc::k_sort_home<<<grid_of(hi - lo, rsc::kSortThreads), rsc::kSortThreads, 0, st>>>(w->sort_order, w->inv, lo, hi - lo);
+        RSC_CUDA(cudaGetLastError());
+        w->launches++;
+        s = permute_slots(w, lo, hi - lo, st);
+        if (s) return s;
+        w->sort_end = std::min(w->sort_end, lo);
+        w->mixed.erase(w->mixed.begin() + (long)q);
+        moved = true;
+    }
+    return moved ? release_main(w) : RSC_OK;
 }
 
 /* Sort when the interval has passed or the state was replaced. */
@@ -1745,6 +1801,9 @@ int rsc_advance_time(rsc_worker *w, const rsc_population *pop, int les_id, const
     if (s) return s;
     s = flush_pending(w);
     if (s) return s;
+    if (pop == nullptr || sim_desc == nullptr) return fail(RSC_ERR_ARG, "population / sim_desc is NULL");
+    s = match_order(w, pop, w->stream);
+    if (s) return s;
     AdvanceArgs a;
     unsigned blocks = 0;
     s = fill_advance_args(w, pop, les_id, sim_desc, a, &blocks);
@@ -1804,6 +1863,8 @@ int rsc_update_debris_rcs(rsc_worker *w, const rsc_population *pop, const float 
     s = flush_pending(w);
     if (s) return s;
     if (pop == nullptr || sim_desc == nullptr) return fail(RSC_ERR_ARG, "population / sim_desc is NULL");
+    s = match_order(w, pop, w->stream);
+    if (s) return s;
     AdvanceArgs a;
     memset(&a, 0, sizeof(a));
     a.pos_in = a.pos = w->pos;
@@ -3052,7 +3113,8 @@ int batch_run_part(rsc_batch *b, int k0, int steps, bool use_graph, float *pulse
             x->sort_due = true;
             x->sig_aux_stale = false;   /* of a pulse that later ones of this run replace */
         }
-        s = maybe_sort(x, &b->pops[i], row[i].sim, b->stream);
+        s = match_order(x, &b->pops[i], b->stream);
+        if (s == RSC_OK) s = maybe_sort(x, &b->pops[i], row[i].sim, b->stream);
         if (s) return s;
         /* the advances write both pairs: scatterers outside the population
          * ranges carry over into the other one */

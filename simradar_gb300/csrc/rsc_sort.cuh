@@ -198,6 +198,13 @@ __global__ void __launch_bounds__(kSortThreads) k_iota(unsigned *a, unsigned lon
     if (s < n) a[s] = (unsigned)s;
 }
 
+/* the order that brings the slots [lo, lo + n) back to the caller's */
+__global__ void __launch_bounds__(kSortThreads) k_sort_home(unsigned *order, const unsigned *inv, unsigned long long lo,
+                                                            unsigned long long n) {
+    const unsigned long long j = (unsigned long long)blockIdx.x * kSortThreads + threadIdx.x;
+    if (j < n) order[j] = inv[lo + j] - (unsigned)lo;
+}
+
 /* caller order <-> slot order for upload and download */
 __global__ void __launch_bounds__(kSortThreads) k_gather16(uint4 *dst, const uint4 *src, const unsigned *inv,
                                                            unsigned long long offset, unsigned long long count) {
