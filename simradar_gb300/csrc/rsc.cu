@@ -419,8 +419,8 @@ int fill_debris(rsc_worker *w, const rsc_population *pop, AdvanceArgs &a, unsign
     return RSC_OK;
 }
 
-/* float4 of the nodes' single-scatterer sums: node_copies() copies */
-constexpr size_t kStrayFloat4s = 1024;
+/* The nodes' single-scatterer sums, 4 doubles a node: node_copies() copies */
+constexpr size_t kStrayNodes = 1024;
 
 /* Gate origins: the FP32 running sum of make_pulse_pass_1 (rs.cl:1214) and
  * the FP64 values range_start + k * range_delta (head and tail). */
@@ -773,7 +773,7 @@ void use_nodes(rsc_worker *w, PulseArgs &P, int mode, bool batch) {
     }
     P.mom_n = n;
     P.node = w->node + (rsc::kNodeMaxN - n);
-    P.stray = reinterpret_cast<float4 *>(w->acc64 + (2 * rsc::node_count(w->G, rsc::kNodeMaxN) + w->G) * 4);
+    P.stray = w->acc64 + (2 * rsc::node_count(w->G, rsc::kNodeMaxN) + w->G) * 4;
     P.lead = ordered ? w->sort_end : 0;
     /* half a gate more than the triangles reach; everything when an antenna
      * weight is not finite, which any range meets, or so large that a term may
@@ -992,7 +992,7 @@ int rsc_worker_malloc(rsc_worker *w, size_t num_scats, float range_start, float 
     RSC_CUDA(cudaMalloc((void **)&w->node, nodes * sizeof(float)));
     /* the pulse kernels' FP64 accumulator (gates; or nodes, or intervals, and then gates);
      * each launch leaves it at zero */
-    const size_t acc_bytes = (2 * nodes + range_count) * 4 * sizeof(double) + kStrayFloat4s * sizeof(float4);
+    const size_t acc_bytes = (2 * nodes + range_count + kStrayNodes) * 4 * sizeof(double);
     RSC_CUDA(cudaMalloc((void **)&w->acc64, acc_bytes));
     RSC_CUDA(cudaMemsetAsync(w->acc64, 0, acc_bytes, w->stream));
     RSC_CUDA(cudaMalloc((void **)&w->counter, sizeof(unsigned)));

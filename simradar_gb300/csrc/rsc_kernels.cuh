@@ -489,7 +489,7 @@ struct PulseArgs {
     double *acc64;       /* G * 4 FP64 accumulators, zero between launches */
     unsigned *counter;
     const float *node;          /* node positions of the gate grid, index 0 at node -mom_n (rsc_nodes.cuh) */
-    float4 *stray;              /* the nodes' sums of single scatterers, zero between launches */
+    double *stray;              /* the nodes' sums of single scatterers, zero between launches */
     float reach_lo2, reach_hi2; /* squared ranges between which a scatterer can reach a gate, with a margin */
     unsigned long long lead;    /* leading scatterers in spatial order */
     unsigned long long *runs;   /* the grouped compensated pulse's run counter, zero between launches (or null) */

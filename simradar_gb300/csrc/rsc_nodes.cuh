@@ -124,7 +124,7 @@ __device__ __forceinline__ float warp_sum4(unsigned lane, float v0, float v1, fl
 /* Nodes of a pulse of G gates: m = -n .. G + n - 1, at index m + n. */
 __host__ __device__ __forceinline__ unsigned node_count(unsigned G, int n) { return G + 2u * (unsigned)n; }
 __host__ __device__ __forceinline__ size_t node_smem_bytes(unsigned G, int n, bool compensated) {
-    return (size_t)node_count(G, n) * (compensated ? 8 : 4) * sizeof(double);
+    return (size_t)node_count(G, n) * (compensated ? 8 * sizeof(double) : 4 * sizeof(double) + sizeof(float));
 }
 
 /* 4 blocks of 256 per SM at 64 registers, nothing spilled.  README scale,
@@ -265,6 +265,25 @@ __device__ __forceinline__ double wide_of(float f) {
     if (HEAD && m >= 0x7f800000u) hi |= 0x7ff00000u;
     return __hiloint2double((int)hi, (int)(b << 29));
 }
+/* The same of a double of FP32's range. */
+__device__ __forceinline__ double wide_scaled(double v) {
+    const unsigned hi = (unsigned)__double2hiint(v), m = hi & 0x7fffffffu;
+    if (m - 0x38100000u >= 0x0fe00000u) return v * (1.0 / kWideScale);   /* beyond FP32's normal numbers */
+    return __hiloint2double((int)(hi - 0x38000000u), __double2loint(v));
+}
+/* And back, as a double-float: 24 bits of head, cut off, and 29 of tail; false
+ * beyond FP32's range. */
+__device__ __forceinline__ bool wide_split(double d, float &h, float &l) {
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+    const unsigned s = hi & 0x80000000u, m = hi & 0x7fffffffu, e = m >> 20;
+    h = __uint_as_float(s | (m << 3) | (lo >> 29));
+    l = e > 23u ? __uint_as_float(s | ((e - 23u) << 23)) * ((float)(lo & 0x1fffffffu) * 0x1p-29f) : 0.0f;
+    return e < 0xffu;
+}
+__device__ __forceinline__ bool not_zero(double d) {
+    return (((unsigned)__double2hiint(d) & 0x7fffffffu) | (unsigned)__double2loint(d)) != 0u;
+}
+
 /* A double-float into a sum in L2 (of 2^-896 times the values), as two
  * reductions: the additions happen there, not in the SM's few FP64 lanes.  (As atomicAdd through a generic
  * pointer each waited for its answer: 3 us per scatterer.) */
@@ -478,22 +497,26 @@ __device__ __forceinline__ int node_interval(const PulseArgs &P, float r) {
     return j > last ? -1 : j;
 }
 
-/* One scatterer, in interval j, by itself: two 16-byte reductions in L2,
- * which nothing waits for. */
-__device__ __forceinline__ void red_add4(float4 *p, float a, float b, float c, float d) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-__device__ __forceinline__ void node_stray(const PulseArgs &P, float4 *stray, int j, float r, const float *v) {
+/* One scatterer, in interval j, by itself: eight FP64 reductions in L2 (scaled
+ * as wide_of), which nothing waits for.  (2,000,000 out of spatial order on 512
+ * gates 1.5 m apart, which all go this way: 799 us; 273 as two reductions of
+ * four FP32 values, whose sums of 1e5 terms lose three digits; 4,082 with every
+ * gate visited.) */
+__device__ __forceinline__ void node_stray(const PulseArgs &P, double *stray, int j, float r, const float *v) {
     const float a = __ldg(P.node + j), b = __ldg(P.node + j + 1), i = 1.0f / (b - a);
     const float wa = (b - r) * i, wb = (r - a) * i;
-    red_add4(stray + j, wa * v[0], wa * v[1], wa * v[2], wa * v[3]);
-    red_add4(stray + j + 1, wb * v[0], wb * v[1], wb * v[2], wb * v[3]);
+    double *o = stray + 4 * (unsigned)j;
+#pragma unroll
+    for (int l = 0; l < 4; l++) {
+        red_add(o + l, wide_of<true>(wa * v[l]));
+        red_add(o + 4 + l, wide_of<true>(wb * v[l]));
+    }
 }
 
 /* A lane's scatterer by itself: to every gate when not finite, nowhere when
  * it reaches none. */
 __device__ __forceinline__ bool sig_finite(const Sig &g) { return fabsf(g.r) < INFINITY && finite4(g.s); }
-__device__ __forceinline__ void node_alone(const PulseArgs &P, const Sig &g, float4 *stray) {
+__device__ __forceinline__ void node_alone(const PulseArgs &P, const Sig &g, double *stray) {
     if (!sig_finite(g)) {
         node_non_finite(P, g.r, g.s[0], g.s[1], g.s[2], g.s[3]);
         return;
@@ -507,7 +530,7 @@ __device__ __forceinline__ void node_alone(const PulseArgs &P, const Sig &g, flo
  * where a good part of the run lies, holds is added to it, and the rest --
  * debris, scatterers respawned elsewhere since the last sort -- one by one. */
 __device__ __forceinline__ void node_settle(const PulseArgs &P, NodeWindow &W, const Sig *g, unsigned in, int part,
-                                            double *bins, float4 *stray, unsigned lane) {
+                                            double *bins, double *stray, unsigned lane) {
     int j[2];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
@@ -610,37 +633,63 @@ __device__ __forceinline__ void node_gates(const PulseArgs &P, double *bins, uns
         if (threadIdx.x == 0) *P.counter = 0u;
         return;
     }
-    float *sums = reinterpret_cast<float *>(bins), *at_node = sums + 4 * nodes;
+    /* each node's sum as a double-float, over bins[o], whose sums are out: the
+     * FP64 units of the one block add 2 numbers a cycle (500,000 scatterers on
+     * 240 gates, 4 pulses: 178 us with FP64 sums here, 170 with these, 167 with
+     * FP32 ones) */
+    float2 *sums = reinterpret_cast<float2 *>(bins);
+    float *at_node = reinterpret_cast<float *>(sums + 4 * nodes);
     const unsigned copies = node_copies(P.G, P.mom_n);
-    const float *stray = reinterpret_cast<const float *>(P.stray);
-    /* the loads of several sums in flight at once: no store between them */
+    bool fits = true;
+    /* the loads of several sums in flight at once: no store or branch between them */
 #pragma unroll 4
     for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) {
-        float v = (float)__ldcg(P.acc64 + o), t = 0.0f;
+        double d[STRAY ? kNodeCopies + 1 : 1];
+        d[0] = __ldcg(P.acc64 + o);
 #pragma unroll
-        for (unsigned c = 0; c < kNodeCopies; c++) {
-            if (STRAY && c < copies) t = t + __ldcg(stray + (size_t)c * 4 * nodes + o);
+        for (unsigned c = 0; STRAY && c < kNodeCopies; c++) {
+            d[c + 1] = c < copies ? __ldcg(P.stray + (size_t)c * 4 * nodes + o) : 0.0;
         }
-        sums[o] = v + t;   /* over bins[o / 2], whose sums are out */
+        float h, l;
+        fits = wide_split(d[0], h, l) && fits;
+#pragma unroll
+        for (unsigned c = 0; STRAY && c < kNodeCopies; c++) {
+            float a, b;
+            fits = wide_split(d[c + 1], a, b) && fits;
+            df_acc(h, l, a, b);
+        }
+        sums[o] = make_float2(h, l);
     }
     for (unsigned o = threadIdx.x; o < nodes; o += blockDim.x) at_node[o] = __ldg(P.node + o);
-    __syncthreads();
+    if (__syncthreads_or(!fits)) {
+        for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) {
+            double v = __ldcg(P.acc64 + o);
+            for (unsigned c = 0; STRAY && c < copies; c++) v = v + __ldcg(P.stray + (size_t)c * 4 * nodes + o);
+            v = v * kWideScale;
+            const float h = (float)v;
+            sums[o] = make_float2(h, fabsf(h) < INFINITY ? (float)(v - (double)h) : 0.0f);
+        }
+        __syncthreads();
+    }
     for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) P.acc64[o] = 0.0;
-    for (unsigned o = threadIdx.x; STRAY && o < nodes * copies; o += blockDim.x) P.stray[o] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (unsigned o = threadIdx.x; STRAY && o < 4 * nodes * copies; o += blockDim.x) P.stray[o] = 0.0;
     const int n = P.mom_n;
     for (unsigned o = threadIdx.x; o < outs; o += blockDim.x) {
         const unsigned k = o >> 2, l = o & 3u;
         const float rk = __ldg(P.rk + k);
-        float sum = 0.0f;
+        float sum = 0.0f, low = 0.0f;
         const unsigned end = min(k + 2u * (unsigned)n + 1u, nodes);
 #pragma unroll 4
         for (unsigned at = k; at < end; at++) {
             const float w = fmaxf(1.0f - fabsf(at_node[at] - rk) * P.rwd[0], 0.0f);
-            sum = fmaf(w, sums[4 * at + l], sum);
+            float a, b;
+            df_mul_pair(sums[4 * at + l].x, sums[4 * at + l].y, w, 0.0f, a, b);
+            df_acc(sum, low, a, b);
         }
+        sum = sum + low;
         const double e = o == threadIdx.x ? e0 : __ldcg(extra + o);
-        if (e != 0.0) {
-            sum = (float)((double)sum + e);
+        if (not_zero(e)) {
+            sum = (float)((double)sum + e);   /* not finite */
             extra[o] = 0.0;
         }
         reinterpret_cast<float *>(P.pulse)[o] = sum;
@@ -656,7 +705,7 @@ __device__ __forceinline__ void node_finish(const PulseArgs &P, double *bins, un
         __syncthreads();
         for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) {
             const double v = bins[o];
-            if (v != 0.0) red_add(P.acc64 + o, v);
+            if (not_zero(v)) red_add(P.acc64 + o, wide_scaled(v));
         }
     }
     node_gates<MODE, true>(P, bins, nblk);
@@ -664,7 +713,7 @@ __device__ __forceinline__ void node_finish(const PulseArgs &P, double *bins, un
 
 /* A run of 64 into the warp's window. */
 __device__ __forceinline__ void node_run(const PulseArgs &P, NodeWindow &W, const float4 *p, const float4 *x, unsigned in,
-                                         int part, double *bins, float4 *stray, unsigned lane) {
+                                         int part, double *bins, double *stray, unsigned lane) {
     Sig g[2];
     bool held[2];
 #pragma unroll
@@ -752,7 +801,7 @@ __device__ __forceinline__ void node_body(const PulseArgs &P, unsigned blk, unsi
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *bins = reinterpret_cast<double *>(smem_raw);
     const unsigned nodes = node_count(P.G, P.mom_n);
-    float4 *stray = P.stray + (size_t)nodes * (blk & (node_copies(P.G, P.mom_n) - 1u));
+    double *stray = P.stray + (size_t)4 * nodes * (blk & (node_copies(P.G, P.mom_n) - 1u));
     if (MODE == 0) {
         for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) bins[o] = 0.0;
         __syncthreads();
@@ -835,7 +884,8 @@ __global__ void __launch_bounds__(kNodeThreads, kCompMinBlocks) k_pulse_nodes_co
  * caller's own buffers, n = 4 100 -> 27.  With 3 and 2 blocks per SM 43 and 56
  * instead of 41. */
 __host__ __device__ __forceinline__ size_t node_any_smem_bytes(unsigned G, int n, int warps) {
-    return (size_t)node_count(G, n) * (1 + 4 * (size_t)warps) * sizeof(float);
+    const size_t own = (size_t)node_count(G, n) * (1 + 4 * (size_t)warps) * sizeof(float), last = node_smem_bytes(G, n, false);
+    return own > last ? own : last;   /* the last block's sums of the nodes take the place of the warps' */
 }
 /* ... while 4 blocks fit an SM with it. */
 constexpr size_t kNodeAnyMost = 54 * 1024;
@@ -900,7 +950,7 @@ __global__ void __launch_bounds__(kNodeThreads, kNodeMinBlocks) k_pulse_nodes_an
         const unsigned at = (o & 3u) * nodes + (o >> 2);
         float v = 0.0f;
         for (unsigned w = 0; w < nwarps; w++) v = v + sums[(size_t)w * 4 * nodes + at];
-        if (v != 0.0f) red_add(P.acc64 + o, (double)v);
+        if (v != 0.0f) red_add(P.acc64 + o, wide_of<true>(v));
     }
     node_gates<0, false>(P, reinterpret_cast<double *>(smem_raw), gridDim.x);
 }
