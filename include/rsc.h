@@ -224,15 +224,23 @@ int rsc_set_fused_step(rsc_worker *w, int enable);
 /* ---- launch-shape autotuning (additive) ----
  * Time the pulse kernel of this worker at each candidate shape (warps per
  * block 4 / 8 / 16 and 1-4 resident blocks per SM) on the current state and
- * keep the fastest for later rsc_make_pulse calls.  sim_desc is the beam to
- * time with; the state is not changed (the pulse is recomputed). */
+ * keep the fastest for later rsc_make_pulse calls of the same kernel: a state
+ * in spatial order (after the first advance) takes another one than a state
+ * just uploaded, and each precision its own; those keep their defaults.
+ * sim_desc is the beam to time with; the state is not changed (the pulse is
+ * recomputed). */
 int rsc_autotune(rsc_worker *w, const float sim_desc[16], int *warps_out, int *blocks_per_sm_out);
 /* Set the pulse kernel's shape directly: warps per block (1-16) and resident
  * blocks per SM (1-4), each capped by what the kernel's shared memory and
  * registers allow; 0 for either returns to the largest that fits.  Fewer
  * pulse blocks per SM leave room for the advance of the same step, which
- * runs beside the pulse on the advance stream. */
+ * runs beside the pulse on the advance stream.  It holds for every pulse
+ * kernel; those that sum on the nodes of the gate grid (a triangle of a whole
+ * number of gate spacings) take at most 8 warps. */
 int rsc_set_pulse_shape(rsc_worker *w, int warps, int blocks_per_sm);
+/* The shape of the latest pulse's launch (0, 0 before one; a small state may
+ * launch fewer blocks than the SMs hold of it). */
+int rsc_get_pulse_shape(rsc_worker *w, int *warps, int *blocks_per_sm);
 /* Background scatterers per thread of the advance (1 or 2; el_atts and
  * bg_atts): with 2 a thread forms two scatterers' steps before storing
  * either, overlapping their dependent loads.  The state is the same. */

@@ -145,6 +145,7 @@ struct rsc_worker {
     uint64_t launches = 0;
     /* pulse launch shape chosen by rsc_autotune (0: default) */
     int tune_warps = 0, tune_per_sm = 0;
+    int tune_for = -1;            /* the pulse kernel they were timed for (kernel_key), -1: set for all */
     int adv_per_thread = 1;   /* background scatterers per advance thread (rsc_set_advance_shape) */
     /* spatial order of the background range (rsc_sort.cuh): perm[slot] is the
      * caller's index, inv[index] the slot; NULL perm = caller's order */
@@ -580,8 +581,14 @@ int node_grid(unsigned long long n, int threads) {
     return (int)std::min<unsigned long long>(std::max<unsigned long long>((n + per_block - 1) / per_block, 1), 1u << 20);
 }
 
+int kernel_key(int mode, int path) { return 8 * mode + path; }
+
 int pulse_geometry(rsc_worker *w, int mode, int path, int mom_n, int *grid, int *threads, size_t *smem) {
-    const int key[6] = {mode, path, (int)w->G, w->tune_warps, w->tune_per_sm, mom_n};
+    /* a shape timed for another kernel (a state out of spatial order, another
+     * precision) says nothing about this one */
+    const bool own = w->tune_for < 0 || w->tune_for == kernel_key(mode, path);
+    const int warps = own ? w->tune_warps : 0, want = own ? w->tune_per_sm : 0;
+    const int key[6] = {mode, path, (int)w->G, warps, want, mom_n};
     if (memcmp(key, w->geo_key, sizeof(key)) == 0) {
         /* same shape as the last launch: no occupancy query per pulse */
         *grid = w->geo_grid;
@@ -590,7 +597,7 @@ int pulse_geometry(rsc_worker *w, int mode, int path, int mom_n, int *grid, int 
         return RSC_OK;
     }
     int per_sm = 1;
-    int s = pulse_shape(mode, false, w->G, w->tune_warps, w->tune_per_sm, &per_sm, threads, smem, path, mom_n);
+    int s = pulse_shape(mode, false, w->G, warps, want, &per_sm, threads, smem, path, mom_n);
     if (s) return s;
     *grid = w->num_sms * per_sm;
     memcpy(w->geo_key, key, sizeof(key));
@@ -2523,6 +2530,14 @@ int rsc_set_pulse_shape(rsc_worker *w, int warps, int blocks_per_sm) {
     }
     w->tune_warps = warps;
     w->tune_per_sm = blocks_per_sm;
+    w->tune_for = -1;
+    return RSC_OK;
+}
+
+int rsc_get_pulse_shape(rsc_worker *w, int *warps, int *blocks_per_sm) {
+    if (w == nullptr) return fail(RSC_ERR_ARG, "worker is NULL");
+    if (warps) *warps = w->geo_threads / 32;
+    if (blocks_per_sm) *blocks_per_sm = w->num_sms ? w->geo_grid / w->num_sms : 0;
     return RSC_OK;
 }
 
@@ -2571,7 +2586,8 @@ int rsc_autotune(rsc_worker *w, const float sim_desc[16], int *warps_out, int *b
                             P.mom_n);
             if (s) return s;
             if (threads != warps * 32 || got != per_sm) continue;   /* shape not reachable */
-            const int grid = w->num_sms * per_sm;
+            int grid = w->num_sms * per_sm;
+            if (pulse_path(P, mode) >= 5) grid = std::min(grid, node_grid(P.n, threads));
             launch_pulse(mode, P, grid, threads, smem, w->stream);
             RSC_CUDA(cudaEventRecord(ev.a, w->stream));
             for (int r = 0; r < kTuneReps; r++) launch_pulse(mode, P, grid, threads, smem, w->stream);
@@ -2593,6 +2609,7 @@ int rsc_autotune(rsc_worker *w, const float sim_desc[16], int *warps_out, int *b
     if (s) return s;
     w->tune_warps = best_w;
     w->tune_per_sm = best_p;
+    w->tune_for = kernel_key(mode, pulse_path(P, mode));
     memcpy(w->last_sim, sim_desc, sizeof(w->last_sim));
     w->have_pulse_desc = true;
     w->sig_aux_stale = true;

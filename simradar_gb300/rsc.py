@@ -107,6 +107,7 @@ def load_library():
         "rsc_get_advance_stream": ([P, ctypes.POINTER(P)], I),
         "rsc_eval_math": ([I, _f32p, _f32p, _f32p, S], I),
         "rsc_autotune": ([P, _f32p, ctypes.POINTER(I), ctypes.POINTER(I)], I),
+        "rsc_get_pulse_shape": ([P, ctypes.POINTER(I), ctypes.POINTER(I)], I),
         "rsc_set_pulse_shape": ([P, I, I], I),
         "rsc_set_advance_shape": ([P, I], I),
         "rsc_set_sort_interval": ([P, I], I),
@@ -373,6 +374,13 @@ class Worker:
         d = f32(sim_desc)
         wv, pv = ctypes.c_int(0), ctypes.c_int(0)
         _check(self._lib.rsc_autotune(self._h, _fp(d), ctypes.byref(wv), ctypes.byref(pv)))
+        return wv.value, pv.value
+
+    @property
+    def pulse_shape(self):
+        """Warps per block and blocks per SM of the latest pulse's launch."""
+        wv, pv = ctypes.c_int(0), ctypes.c_int(0)
+        _check(self._lib.rsc_get_pulse_shape(self._h, ctypes.byref(wv), ctypes.byref(pv)))
         return wv.value, pv.value
 
     def set_pulse_shape(self, warps, blocks_per_sm):
