@@ -314,7 +314,8 @@ int rsc_batch_synchronize(rsc_batch *b);
 int rsc_batch_set_les_async(rsc_batch *b, int index, int slot, const float *uvwt4, const float *cpxx4, uint32_t nx,
                             uint32_t ny, uint32_t nz);
 /* The persistent form (additive, off by default): rsc_batch_run and
- * rsc_batch_run_async then run all steps of every instance in one launch.
+ * rsc_batch_run_async then run all steps of every instance in one launch (of
+ * each part, where the run goes in parts).
  * Each block owns fixed segments of the instances' scatterers (cut on the
  * host to equal cost) and, step after step, forms their share of the pulse
  * and advances them; no block waits for another (the pulses of different

@@ -3061,7 +3061,7 @@ int batch_persist_prepare(rsc_batch *b, int steps) {
     return RSC_OK;
 }
 
-/* Every step of the run in one launch (after zeroing its accumulators). */
+/* Every step of a part of the run in one launch (after zeroing its accumulators). */
 int batch_persist_launch(rsc_batch *b, int steps) {
     const size_t n = b->w.size();
     const size_t slots = (size_t)steps * n;
@@ -3145,7 +3145,8 @@ int batch_run_part(rsc_batch *b, int k0, int steps, bool use_graph, float *pulse
                              b->stream));
     RSC_CUDA(cudaEventRecord(b->ev_h2d, b->stream));
     if (b->persist_now) {
-        s = batch_persist_prepare(b, steps);
+        /* the segments are those of the whole run, its first part the longest */
+        if (k0 == 0) s = batch_persist_prepare(b, steps);
         if (s == RSC_OK) s = batch_persist_launch(b, steps);
         if (s) return s;
     } else if (use_graph) {

@@ -206,10 +206,10 @@ k_pulse_batch(const PulseArgs *inst, const BatchStep *steps, const unsigned *pre
     }
 }
 
-/* ---- every step of a run in one launch (the persistent form) ----
+/* ---- every step of a run's part in one launch (the persistent form) ----
  * Each block owns a fixed list of segments -- contiguous index ranges of an
  * instance, cut by the host so that every block carries the same cost --
- * and runs every step of the run on them: the segment's share of the
+ * and runs every step of the part on them: the segment's share of the
  * instance's pulse (its bins summed into that step's accumulator of the
  * instance, the last of the instance's blocks converting it), then the
  * advance of the same scatterers into the step's other pos / rcs pair.  The

@@ -444,7 +444,7 @@ class Batch:
         return t.value, p.value
 
     def set_persistent(self, enable):
-        """Run every step of a run in one launch (rsc_batch_set_persistent)."""
+        """Run every step of a run's part in one launch (rsc_batch_set_persistent)."""
         _check(self._lib.rsc_batch_set_persistent(self._h, 1 if enable else 0))
 
     def autotune(self, sim_descs):
