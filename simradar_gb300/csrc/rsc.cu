@@ -2076,7 +2076,7 @@ struct rsc_batch {
     int device = 0;
     int num_sms = 0;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ev_join = nullptr, ev_h2d = nullptr, ev_done = nullptr;
+    cudaEvent_t ev_join = nullptr, ev_done = nullptr;
     /* the debris kernel beside the background kernel (high priority) */
     cudaStream_t side = nullptr;
     cudaEvent_t fork_ev = nullptr, side_ev = nullptr;
@@ -2112,7 +2112,15 @@ struct rsc_batch {
     size_t pulse_smem = 0;
     /* per-step descriptors (pinned on the host) and the pulses of a run */
     int cap_steps = 0;
-    rsc::BatchStep *h_steps = nullptr;
+    /* two host sides, so that the next run's are filled while this run's last
+     * part has not been copied yet: the steps' rows, and a slot of launch
+     * descriptors for every part */
+    rsc::BatchStep *h_rows[2] = {nullptr, nullptr};
+    unsigned char *h_desc[2] = {nullptr, nullptr};
+    size_t desc_slots = 0, desc_at = 0;
+    int side_at = 0;
+    cudaEvent_t ev_h2d[2] = {nullptr, nullptr};   /* the side's copies so far */
+    rsc::BatchStep *h_steps = nullptr;   /* of side_at */
     rsc::BatchStep *d_steps = nullptr;
     float4 *d_out = nullptr;
     cudaGraphExec_t graph = nullptr;
@@ -2155,24 +2163,63 @@ void batch_drop_graph(rsc_batch *b) {
 }
 
 /* Room for `steps` steps of per-step descriptors and pulses. */
-int batch_reserve(rsc_batch *b, int steps) {
-    if (steps <= b->cap_steps) return RSC_OK;
+/* Steps that a run of `steps` takes between sorts of its instances: about equal
+ * parts (one graph serves all but a shorter last one) of at most half the
+ * shortest interval that a worker asked for, 64 or more; the whole run when a
+ * worker keeps the caller's order.  64 instances, runs of 500 steps: 17,141
+ * pulses/s sorted between runs only, 18,638 in parts of up to 128, 19,306 of up
+ * to 64, 19,307 of up to 32. */
+constexpr uint64_t kBatchPart = 64;
+int batch_part(rsc_batch *b, int steps) {
+    uint64_t most = UINT64_MAX;
+    for (rsc_worker *x : b->w) {
+        if (x->sort_interval <= 0) return steps;
+        most = std::min(most, (uint64_t)x->sort_interval);
+    }
+    most = std::max(most / 2, kBatchPart);
+    const uint64_t parts = ((uint64_t)steps + most - 1) / most;
+    return (int)(((uint64_t)steps + parts - 1) / parts);
+}
+
+size_t batch_desc_bytes(const rsc_batch *b) {
+    const size_t n = b->w.size();
+    return (n * (sizeof(rsc::BatchAdvance) + sizeof(PulseArgs)) + 3 * (n + 1) * sizeof(unsigned) + 15) / 16 * 16;
+}
+
+/* Room for a run of `steps` in `parts` parts. */
+int batch_reserve(rsc_batch *b, int steps, size_t parts) {
+    if (steps <= b->cap_steps && parts <= b->desc_slots) return RSC_OK;
     RSC_CUDA(cudaStreamSynchronize(b->stream));
+    const size_t n = b->w.size();
+    cudaError_t e = cudaSuccess;
+    if (parts > b->desc_slots) {
+        b->desc_slots = 0;
+        for (unsigned char *&d : b->h_desc) {
+            if (d) cudaFreeHost(d);
+            d = nullptr;
+            if (e == cudaSuccess) e = cudaMallocHost((void **)&d, parts * batch_desc_bytes(b));
+        }
+        if (e != cudaSuccess) return cuda_fail(RSC_ERR_NOMEM, "batch descriptors for %zu parts: %s", parts, cudaGetErrorString(e));
+        b->desc_slots = parts;
+    }
+    if (steps <= b->cap_steps) return RSC_OK;
     batch_drop_graph(b);
-    if (b->h_steps) cudaFreeHost(b->h_steps);
     free_ptr(b->d_steps);
     free_ptr(b->d_out);
-    b->h_steps = nullptr;
     b->d_steps = nullptr;
     b->d_out = nullptr;
     b->cap_steps = 0;
-    const size_t n = b->w.size();
     const size_t rows = (size_t)steps * n;
-    cudaError_t e = cudaMallocHost((void **)&b->h_steps, rows * sizeof(rsc::BatchStep));
+    for (rsc::BatchStep *&h : b->h_rows) {
+        if (h) cudaFreeHost(h);
+        h = nullptr;
+        if (e == cudaSuccess) e = cudaMallocHost((void **)&h, rows * sizeof(rsc::BatchStep));
+        if (e == cudaSuccess) memset(h, 0, rows * sizeof(rsc::BatchStep));
+    }
+    b->h_steps = b->h_rows[b->side_at];
     if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_steps, rows * sizeof(rsc::BatchStep));
     if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_out, rows * b->Gmax * sizeof(float4));
     if (e != cudaSuccess) return cuda_fail(RSC_ERR_NOMEM, "batch buffers for %d steps: %s", steps, cudaGetErrorString(e));
-    memset(b->h_steps, 0, rows * sizeof(rsc::BatchStep));
     RSC_CUDA(cudaMemsetAsync(b->d_out, 0, rows * b->Gmax * sizeof(float4), b->stream));
     b->cap_steps = steps;
     return RSC_OK;
@@ -2292,15 +2339,26 @@ int batch_prepare(rsc_batch *b, const rsc::BatchStep *row, int steps) {
     b->pulse_threads = threads;
     b->pulse_smem = smem;
     b->pulse_per_sm = per_sm;
-    /* pageable sources: each copy has taken its bytes when the call returns */
-    RSC_CUDA(cudaMemcpyAsync(b->d_adv, b->h_adv.data(), n * sizeof(rsc::BatchAdvance), cudaMemcpyHostToDevice, b->stream));
-    RSC_CUDA(cudaMemcpyAsync(b->d_pulse, b->h_pulse.data(), n * sizeof(PulseArgs), cudaMemcpyHostToDevice, b->stream));
-    RSC_CUDA(cudaMemcpyAsync(b->d_rain_prefix, b->h_rain_prefix.data(), (n + 1) * sizeof(unsigned),
-                             cudaMemcpyHostToDevice, b->stream));
-    RSC_CUDA(cudaMemcpyAsync(b->d_deb_prefix, b->h_deb_prefix.data(), (n + 1) * sizeof(unsigned),
-                             cudaMemcpyHostToDevice, b->stream));
-    RSC_CUDA(cudaMemcpyAsync(b->d_pulse_prefix, b->h_pulse_prefix.data(), (n + 1) * sizeof(unsigned),
-                             cudaMemcpyHostToDevice, b->stream));
+    /* from page-locked memory, which a copy reads later: a slot for each part
+     * of a run (pageable descriptors of 40 instances held the host up until
+     * the part before was done) */
+    if (b->desc_at >= b->desc_slots) {
+        RSC_CUDA(cudaEventSynchronize(b->ev_h2d[b->side_at]));
+        b->desc_at = 0;
+    }
+    unsigned char *h = b->h_desc[b->side_at] + b->desc_at++ * batch_desc_bytes(b);
+    const auto send = [&](void *dst, const void *src, size_t bytes) {
+        memcpy(h, src, bytes);
+        const cudaError_t e = cudaMemcpyAsync(dst, h, bytes, cudaMemcpyHostToDevice, b->stream);
+        h += bytes;
+        return e;
+    };
+    RSC_CUDA(send(b->d_adv, b->h_adv.data(), n * sizeof(rsc::BatchAdvance)));
+    RSC_CUDA(send(b->d_pulse, b->h_pulse.data(), n * sizeof(PulseArgs)));
+    RSC_CUDA(send(b->d_rain_prefix, b->h_rain_prefix.data(), (n + 1) * sizeof(unsigned)));
+    RSC_CUDA(send(b->d_deb_prefix, b->h_deb_prefix.data(), (n + 1) * sizeof(unsigned)));
+    RSC_CUDA(send(b->d_pulse_prefix, b->h_pulse_prefix.data(), (n + 1) * sizeof(unsigned)));
+    RSC_CUDA(cudaEventRecord(b->ev_h2d[b->side_at], b->stream));
     return RSC_OK;
 }
 
@@ -2480,7 +2538,10 @@ void batch_swap_pairs(rsc_batch *b, int steps) {
 /* Copy steps' descriptors into the pinned table, checking them. */
 int batch_fill_steps(rsc_batch *b, int steps, const float *sim_descs, const int *les_ids) {
     const size_t n = b->w.size();
-    RSC_CUDA(cudaEventSynchronize(b->ev_h2d));   /* the last run's copy of the table has been taken */
+    b->side_at ^= 1;
+    RSC_CUDA(cudaEventSynchronize(b->ev_h2d[b->side_at]));   /* the copies of the run before the last have been taken */
+    b->h_steps = b->h_rows[b->side_at];
+    b->desc_at = 0;
     for (int k = 0; k < steps; k++) {
         for (size_t i = 0; i < n; i++) {
             const size_t r = (size_t)k * n + i;
@@ -2646,7 +2707,9 @@ int rsc_batch_create(rsc_worker *const *workers, int count, rsc_batch **out) {
     const int prio_main = prio_greatest < prio_least ? prio_greatest + 1 : prio_greatest;
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->stream, cudaStreamNonBlocking, prio_main);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_h2d, cudaEventDisableTiming);
+    for (cudaEvent_t &v : b->ev_h2d) {
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
+    }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->copy_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&b->side, cudaStreamNonBlocking, prio_greatest);
@@ -2683,7 +2746,10 @@ int rsc_batch_free(rsc_batch *b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     batch_drop_graph(b);
-    if (b->h_steps) cudaFreeHost(b->h_steps);
+    for (int k = 0; k < 2; k++) {
+        if (b->h_rows[k]) cudaFreeHost(b->h_rows[k]);
+        if (b->h_desc[k]) cudaFreeHost(b->h_desc[k]);
+    }
     free_ptr(b->d_steps);
     free_ptr(b->d_out);
     free_ptr(b->d_adv);
@@ -2721,7 +2787,9 @@ int rsc_batch_free(rsc_batch *b) {
     }
     if (b->ev_afork) cudaEventDestroy(b->ev_afork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
-    if (b->ev_h2d) cudaEventDestroy(b->ev_h2d);
+    for (cudaEvent_t v : b->ev_h2d) {
+        if (v) cudaEventDestroy(v);
+    }
     if (b->ev_done) cudaEventDestroy(b->ev_done);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
@@ -2879,7 +2947,7 @@ int rsc_batch_autotune(rsc_batch *b, const float *sim_descs) {
     int s = check_batch(b);
     if (s) return s;
     if (sim_descs == nullptr) return fail(RSC_ERR_ARG, "sim_descs is NULL");
-    s = batch_reserve(b, 1);
+    s = batch_reserve(b, 1, 8);
     if (s) return s;
     s = batch_fill_steps(b, 1, sim_descs, nullptr);
     if (s) return s;
@@ -2888,7 +2956,7 @@ int rsc_batch_autotune(rsc_batch *b, const float *sim_descs) {
     const size_t n = b->w.size();
     batch_fill_pairs(b, b->h_steps, 1);
     RSC_CUDA(cudaMemcpyAsync(b->d_steps, b->h_steps, n * sizeof(rsc::BatchStep), cudaMemcpyHostToDevice, b->stream));
-    RSC_CUDA(cudaEventRecord(b->ev_h2d, b->stream));
+    RSC_CUDA(cudaEventRecord(b->ev_h2d[b->side_at], b->stream));
     EventPair ev;
     RSC_CUDA(ev.init());
     float best = INFINITY;
@@ -3099,24 +3167,6 @@ int batch_persist_launch(rsc_batch *b, int steps) {
     return RSC_OK;
 }
 
-/* Steps that a run of `steps` takes between sorts of its instances: about equal
- * parts (one graph serves all but a shorter last one) of at most half the
- * shortest interval that a worker asked for, 64 or more; the whole run when a
- * worker keeps the caller's order.  64 instances, runs of 500 steps: 17,141
- * pulses/s sorted between runs only, 18,638 in parts of up to 128, 19,306 of up
- * to 64, 19,307 of up to 32. */
-constexpr uint64_t kBatchPart = 64;
-int batch_part(rsc_batch *b, int steps) {
-    uint64_t most = UINT64_MAX;
-    for (rsc_worker *x : b->w) {
-        if (x->sort_interval <= 0) return steps;
-        most = std::min(most, (uint64_t)x->sort_interval);
-    }
-    most = std::max(most / 2, kBatchPart);
-    const uint64_t parts = ((uint64_t)steps + most - 1) / most;
-    return (int)(((uint64_t)steps + parts - 1) / parts);
-}
-
 /* Steps [k0, k0 + steps) of a run: the sort when it is due, the descriptors,
  * the launches and the copy of their pulses.  The device's tables and pulses
  * are the same for every part, in stream order; the host's rows are not. */
@@ -3143,7 +3193,7 @@ int batch_run_part(rsc_batch *b, int k0, int steps, bool use_graph, float *pulse
     batch_fill_pairs(b, row, steps);
     RSC_CUDA(cudaMemcpyAsync(b->d_steps, row, (size_t)steps * n * sizeof(rsc::BatchStep), cudaMemcpyHostToDevice,
                              b->stream));
-    RSC_CUDA(cudaEventRecord(b->ev_h2d, b->stream));
+    RSC_CUDA(cudaEventRecord(b->ev_h2d[b->side_at], b->stream));
     if (b->persist_now) {
         /* the segments are those of the whole run, its first part the longest */
         if (k0 == 0) s = batch_persist_prepare(b, steps);
@@ -3175,7 +3225,8 @@ int batch_run(rsc_batch *b, int steps, const float *sim_descs, const int *les_id
     if (s) return s;
     if (steps < 1) return fail(RSC_ERR_ARG, "steps %d", steps);
     if (sim_descs == nullptr || les_ids == nullptr) return fail(RSC_ERR_ARG, "sim_descs / les_ids is NULL");
-    s = batch_reserve(b, steps);
+    const int part = batch_part(b, steps);
+    s = batch_reserve(b, steps, ((size_t)steps + part - 1) / part);
     if (s) return s;
     s = batch_fill_steps(b, steps, sim_descs, les_ids);
     if (s) return s;
@@ -3195,7 +3246,6 @@ int batch_run(rsc_batch *b, int steps, const float *sim_descs, const int *les_id
         rsc_worker *x = b->w[q / 2];
         if (used[q] && x->les_wait[q & 1]) RSC_CUDA(cudaStreamWaitEvent(b->stream, x->les_ready[q & 1], 0));
     }
-    const int part = batch_part(b, steps);
     for (int k0 = 0; k0 < steps; k0 += part) {
         s = batch_run_part(b, k0, std::min(part, steps - k0), use_graph != 0 && steps - k0 >= part, pulses_out);
         if (s) return s;

@@ -45,3 +45,11 @@ def queued(backend, persistent, runs, steps=500, instances=4):
 def test_persistent_run_is_queued(backend):
     calls, total = queued(backend, True, 1)
     assert calls[0] < 0.5 * total, (calls, total)
+
+
+@pytest.mark.parametrize("instances,steps", [(4, 500), (40, 100)])
+def test_second_run_is_queued_behind_the_first(backend, instances, steps):
+    """One run may wait in the queue behind the one under way: the call that
+    queues it does not wait for parts of the first."""
+    calls, total = queued(backend, False, 2, steps, instances)
+    assert sum(calls) < 0.5 * total, (calls, total)
