@@ -273,8 +273,12 @@ int rsc_batch_set_precision(rsc_batch *b, int mode);
  * given per-instance sim_descs (count x 16 floats, LES slot 0), then the
  * background advance's shape (threads per block 64 / 128 / 256, with every
  * block that fits resident or half of them) by timing it beside that pulse
- * on scratch copies of the arrays it updates in place.  The state is not
- * changed. */
+ * on scratch copies of the arrays it updates in place.  The pulse is the form
+ * that a long run takes: on the nodes of the gate grid (timed beside the
+ * advance) when every instance has 256 scatterers or more, keeps a spatial
+ * order and has a triangle of a whole number of gate spacings, else gate by
+ * gate (timed alone); the other form keeps its default shape.  The instances
+ * are put in spatial order; the state is not changed. */
 int rsc_batch_autotune(rsc_batch *b, const float *sim_descs);
 /* Set the batched background advance's shape directly: threads per block
  * (64, 128 or 256) and resident blocks per SM (0: as many as fit). */
@@ -337,6 +341,8 @@ int rsc_batch_launch_count(rsc_batch *b, uint64_t *count);
 int rsc_batch_get_stream(rsc_batch *b, void **stream);
 /* The pulse shape chosen by rsc_batch_autotune (0, 0 before it runs). */
 int rsc_batch_get_shape(rsc_batch *b, int *warps, int *blocks_per_sm);
+/* The shape of the latest run's pulses (0, 0 before one). */
+int rsc_batch_get_pulse_shape(rsc_batch *b, int *warps, int *blocks_per_sm);
 
 /* ---- initial state (additive) ----
  * The scatterers RS_populate (rs.c:4568-4814) makes from RS_set_random_seed:

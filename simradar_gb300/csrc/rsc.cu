@@ -728,10 +728,12 @@ double window_margin(double drift, float range_start, float range_delta, uint32_
 }
 
 /* Advances since its sort up to which a state counts as in spatial order, and
- * the most steps a batch, which sorts between runs only, takes through the node
- * sums: as runs of 64 spread over more intervals, their windows move more and
- * the sums gate by gate become the faster (64 instances, compensated, runs of
- * 500 steps: 14,581 pulses/s on the nodes, 17,141 gate by gate).  The default interval of sorts is 128. */
+ * the longest part of a batch's run (batch_part: half the sort interval, 64 steps
+ * by default) that goes through the node sums: as runs of 64 spread over more
+ * intervals, their windows move more and the sums gate by gate become the
+ * faster (64 instances, compensated, 500 steps without a sort between: 14,581
+ * pulses/s on the nodes, 17,141 gate by gate).  The default interval of sorts
+ * is 128. */
 constexpr uint64_t kOrderedSteps = 256;
 constexpr int kNodeBatchSteps = 128;
 
@@ -2090,6 +2092,8 @@ struct rsc_batch {
     int mode = RSC_PULSE_PLAIN;
     uint32_t Gmax = 0;
     int tune_warps = 0, tune_per_sm = 0;
+    bool tuning = false;   /* rsc_batch_autotune tries them */
+    int tune_nodes = -1;   /* the pulse's form they were timed for: node sums 1, gate by gate 0 */
     /* background advance shape: threads per block and the shared-memory
      * bytes each block asks for, which limits the resident blocks per SM
      * (0: as many as fit) */
@@ -2225,9 +2229,8 @@ int batch_reserve(rsc_batch *b, int steps, size_t parts) {
     return RSC_OK;
 }
 
-/* Stands for a run of any length: the shapes that are timed are the ones of
- * the sums gate by gate, which long runs take. */
-constexpr int kTuneSteps = 1 << 30;
+/* The length of a part of a long run: what a shape is timed for. */
+int batch_tune_steps(rsc_batch *b) { return batch_part(b, 1 << 30); }
 
 /* Build every instance's descriptors for the beam / concept of `row` (one
  * BatchStep per instance) for a run of `steps` and the block prefixes; upload them.  A change of
@@ -2305,8 +2308,9 @@ int batch_prepare(rsc_batch *b, const rsc::BatchStep *row, int steps) {
         }
         max_n = 0;
     }
-    /* the node sums at their own shape: the tuned one is of the other form */
-    s = pulse_shape(b->mode, true, b->Gmax, nodes ? 0 : b->tune_warps, nodes ? 0 : b->tune_per_sm, &per_sm, &threads,
+    /* each form at its own shape: one timed for the other says nothing about it */
+    const bool tuned = b->tuning || b->tune_nodes == (nodes ? 1 : 0);
+    s = pulse_shape(b->mode, true, b->Gmax, tuned ? b->tune_warps : 0, tuned ? b->tune_per_sm : 0, &per_sm, &threads,
                     &smem, nodes ? 5 : 0, max_n);
     if (s) return s;
     const double total = (double)b->num_sms * per_sm;
@@ -2823,14 +2827,23 @@ int rsc_batch_set_precision(rsc_batch *b, int mode) {
 
 namespace {
 
-/* The batched background advance's shape, timed as one step beside the
- * batched pulse: threads per block 64 / 128 / 256, each with every block
- * that fits resident and with half of them (shared memory asked for per
- * block).  The advance writes the step's other pos / rcs pair, which the
- * next run overwrites, and the arrays it updates in place (vel, rnd) are
- * scratch copies here, so the state is not changed.  Without the memory for
- * the copies the shape stays as it was. */
-int batch_tune_advance(rsc_batch *b) {
+/* Scratch copies for timing a batched step: the advance writes the step's other
+ * pos / rcs pair, which the next run overwrites, and the arrays it updates in
+ * place (vel, rnd) are copies here, so the state is not changed.  `adv` stays
+ * NULL without the memory for them, or without an advance to time. */
+struct BatchScratch {
+    float4 *vel = nullptr;
+    uint4 *rnd = nullptr;
+    rsc::BatchAdvance *adv = nullptr;
+    ~BatchScratch() {
+        free_ptr(vel);
+        free_ptr(rnd);
+        free_ptr(adv);
+    }
+};
+
+/* After a batch_prepare (the instances' descriptors). */
+int batch_tune_scratch(rsc_batch *b, BatchScratch &c) {
     const size_t n = b->w.size();
     if (b->rain_blocks == 0) return RSC_OK;
     std::vector<size_t> off(n);
@@ -2839,80 +2852,107 @@ int batch_tune_advance(rsc_batch *b) {
         off[i] = total;
         total += b->w[i]->numel;
     }
-    float4 *svel = nullptr;
-    uint4 *srnd = nullptr;
-    rsc::BatchAdvance *sadv = nullptr;
-    cudaError_t e = cudaMalloc((void **)&svel, total * sizeof(float4));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&srnd, total * sizeof(uint4));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&sadv, n * sizeof(rsc::BatchAdvance));
+    cudaError_t e = cudaMalloc((void **)&c.vel, total * sizeof(float4));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&c.rnd, total * sizeof(uint4));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&c.adv, n * sizeof(rsc::BatchAdvance));
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
-        free_ptr(svel);
-        free_ptr(srnd);
+        c.adv = nullptr;
         return RSC_OK;
     }
     std::vector<rsc::BatchAdvance> adv(b->h_adv);
-    int s = RSC_OK;
-    for (size_t i = 0; i < n && s == RSC_OK; i++) {
+    for (size_t i = 0; i < n; i++) {
         rsc_worker *x = b->w[i];
-        adv[i].a.vel = svel + off[i];
-        adv[i].a.rnd = srnd + off[i];
-        if (cudaMemcpyAsync(svel + off[i], x->vel, x->numel * sizeof(float4), cudaMemcpyDeviceToDevice, b->stream) !=
-                cudaSuccess ||
-            cudaMemcpyAsync(srnd + off[i], x->rnd, x->numel * sizeof(uint4), cudaMemcpyDeviceToDevice, b->stream) !=
-                cudaSuccess) {
-            s = cuda_fail(RSC_ERR_CUDA, "advance tuning copies failed");
+        adv[i].a.vel = c.vel + off[i];
+        adv[i].a.rnd = c.rnd + off[i];
+        RSC_CUDA(cudaMemcpyAsync(c.vel + off[i], x->vel, x->numel * sizeof(float4), cudaMemcpyDeviceToDevice, b->stream));
+        RSC_CUDA(cudaMemcpyAsync(c.rnd + off[i], x->rnd, x->numel * sizeof(uint4), cudaMemcpyDeviceToDevice, b->stream));
+    }
+    RSC_CUDA(cudaMemcpyAsync(c.adv, adv.data(), n * sizeof(rsc::BatchAdvance), cudaMemcpyHostToDevice, b->stream));
+    RSC_CUDA(cudaStreamSynchronize(b->stream));
+    return RSC_OK;
+}
+
+/* Milliseconds of kTuneReps steps (the pulse, and beside it the background
+ * advance where there is scratch for it) at the prepared shapes. */
+int batch_time_step(rsc_batch *b, const rsc::BatchAdvance *adv, EventPair &ev, float *ms) {
+    for (int r = 0; r <= kTuneReps; r++) {
+        if (r == 1) RSC_CUDA(cudaEventRecord(ev.a, b->stream));
+        if (adv) {
+            RSC_CUDA(cudaEventRecord(b->ev_afork, b->stream));
+            RSC_CUDA(cudaStreamWaitEvent(b->adv, b->ev_afork, 0));
+        }
+        RSC_CUDA(batch_launch_pulse(b, 0));
+        b->launches++;
+        if (adv) {
+            RSC_CUDA(batch_launch_rain(b, adv, b->d_steps));
+            RSC_CUDA(cudaEventRecord(b->ev_ba[0], b->adv));
+            RSC_CUDA(cudaStreamWaitEvent(b->stream, b->ev_ba[0], 0));
+            b->launches++;
         }
     }
-    if (s == RSC_OK && cudaMemcpyAsync(sadv, adv.data(), n * sizeof(rsc::BatchAdvance), cudaMemcpyHostToDevice,
-                                       b->stream) != cudaSuccess) {
-        s = cuda_fail(RSC_ERR_CUDA, "advance tuning arguments");
+    RSC_CUDA(cudaEventRecord(ev.b, b->stream));
+    RSC_CUDA(cudaEventSynchronize(ev.b));
+    RSC_CUDA(cudaEventElapsedTime(ms, ev.a, ev.b));
+    return RSC_OK;
+}
+
+/* The batched pulse's shape.  Gate by gate the pulse is timed alone; through
+ * the node sums as a step, since fewer of its blocks leave the advance beside
+ * it its share of an SM. */
+int batch_tune_pulse(rsc_batch *b, const BatchScratch &c, EventPair &ev) {
+    float best = INFINITY;
+    int best_w = 0, best_p = 0;
+    for (int warps : kTuneWarps) {
+        for (int per_sm = 1; per_sm <= 4; per_sm++) {
+            b->tune_warps = warps;
+            b->tune_per_sm = per_sm;
+            int s = batch_prepare(b, b->h_steps, batch_tune_steps(b));
+            if (s) return s;
+            if (b->pulse_threads != warps * 32 || b->pulse_per_sm != per_sm) continue;   /* not reachable */
+            float ms = 0.0f;
+            s = batch_time_step(b, b->nodes ? c.adv : nullptr, ev, &ms);
+            if (s) return s;
+            if (ms < best) {
+                best = ms;
+                best_w = warps;
+                best_p = per_sm;
+            }
+        }
     }
-    EventPair ev;
-    if (s == RSC_OK && ev.init() != cudaSuccess) s = cuda_fail(RSC_ERR_CUDA, "advance tuning events");
+    b->tune_warps = best_w;
+    b->tune_per_sm = best_p;
+    b->tune_nodes = b->nodes ? 1 : 0;
+    return RSC_OK;
+}
+
+/* The batched background advance's shape, timed as one step beside the
+ * batched pulse: threads per block 64 / 128 / 256, each with every block
+ * that fits resident and with half of them (shared memory asked for per
+ * block).  Without the memory for the scratch copies the shape stays as it
+ * was. */
+int batch_tune_advance(rsc_batch *b, const BatchScratch &c, EventPair &ev) {
+    if (c.adv == nullptr) return RSC_OK;
     float best = INFINITY;
     int best_t = b->adv_threads, best_p = b->adv_per_sm;
     const int shapes[6][2] = {{128, 0}, {64, 0}, {256, 0}, {128, 8}, {64, 16}, {256, 4}};
-    for (int c = 0; c < 6 && s == RSC_OK; c++) {
-        b->adv_threads = shapes[c][0];
-        b->adv_per_sm = shapes[c][1];
-        s = batch_advance_smem(b, b->adv_threads, b->adv_per_sm, &b->adv_smem);
-        if (s == RSC_OK) s = batch_prepare(b, b->h_steps, kTuneSteps);
-        if (s) break;
+    for (int k = 0; k < 6; k++) {
+        b->adv_threads = shapes[k][0];
+        b->adv_per_sm = shapes[k][1];
+        int s = batch_advance_smem(b, b->adv_threads, b->adv_per_sm, &b->adv_smem);
+        if (s == RSC_OK) s = batch_prepare(b, b->h_steps, batch_tune_steps(b));
         float ms = 0.0f;
-        for (int r = 0; r <= kTuneReps && s == RSC_OK; r++) {
-            cudaError_t q = cudaEventRecord(r == 1 ? ev.a : b->ev_afork, b->stream);
-            if (r == 1 && q == cudaSuccess) q = cudaEventRecord(b->ev_afork, b->stream);
-            if (q == cudaSuccess) q = cudaStreamWaitEvent(b->adv, b->ev_afork, 0);
-            if (q == cudaSuccess) q = batch_launch_pulse(b, 0);
-            if (q == cudaSuccess) q = batch_launch_rain(b, sadv, b->d_steps);
-            if (q == cudaSuccess) q = cudaEventRecord(b->ev_ba[0], b->adv);
-            if (q == cudaSuccess) q = cudaStreamWaitEvent(b->stream, b->ev_ba[0], 0);
-            if (q != cudaSuccess) s = cuda_fail(RSC_ERR_CUDA, "advance tuning step: %s", cudaGetErrorString(q));
-            b->launches += 2;
-        }
-        if (s) break;
-        if (cudaEventRecord(ev.b, b->stream) != cudaSuccess || cudaEventSynchronize(ev.b) != cudaSuccess ||
-            cudaEventElapsedTime(&ms, ev.a, ev.b) != cudaSuccess) {
-            s = cuda_fail(RSC_ERR_CUDA, "advance tuning timing");
-            break;
-        }
+        if (s == RSC_OK) s = batch_time_step(b, c.adv, ev, &ms);
+        if (s) return s;
         if (ms < best) {
             best = ms;
-            best_t = shapes[c][0];
-            best_p = shapes[c][1];
+            best_t = shapes[k][0];
+            best_p = shapes[k][1];
         }
     }
-    (void)cudaStreamSynchronize(b->stream);
-    free_ptr(svel);
-    free_ptr(srnd);
-    free_ptr(sadv);
-    if (s) return s;
     b->adv_threads = best_t;
     b->adv_per_sm = best_p;
-    s = batch_advance_smem(b, best_t, best_p, &b->adv_smem);
-    if (s == RSC_OK) s = batch_prepare(b, b->h_steps, kTuneSteps);
-    return s;
+    return batch_advance_smem(b, best_t, best_p, &b->adv_smem);
 }
 
 }  // namespace
@@ -2947,6 +2987,7 @@ int rsc_batch_autotune(rsc_batch *b, const float *sim_descs) {
     int s = check_batch(b);
     if (s) return s;
     if (sim_descs == nullptr) return fail(RSC_ERR_ARG, "sim_descs is NULL");
+    if (!b->have_pops) return fail(RSC_ERR_STATE, "rsc_batch_set_populations has not been called");
     s = batch_reserve(b, 1, 8);
     if (s) return s;
     s = batch_fill_steps(b, 1, sim_descs, nullptr);
@@ -2954,43 +2995,39 @@ int rsc_batch_autotune(rsc_batch *b, const float *sim_descs) {
     s = batch_join_workers(b);
     if (s) return s;
     const size_t n = b->w.size();
+    for (size_t i = 0; i < n; i++) {
+        /* in the order that a run's pulses find; the advance that is timed
+         * overwrites the pair of the latest pulse */
+        rsc_worker *x = b->w[i];
+        s = match_order(x, &b->pops[i], b->stream);
+        if (s == RSC_OK) s = settle_sig_aux(x, b->stream);
+        if (s == RSC_OK) s = maybe_sort(x, &b->pops[i], b->h_steps[i].sim, b->stream);
+        if (s) return s;
+    }
     batch_fill_pairs(b, b->h_steps, 1);
     RSC_CUDA(cudaMemcpyAsync(b->d_steps, b->h_steps, n * sizeof(rsc::BatchStep), cudaMemcpyHostToDevice, b->stream));
     RSC_CUDA(cudaEventRecord(b->ev_h2d[b->side_at], b->stream));
     EventPair ev;
     RSC_CUDA(ev.init());
-    float best = INFINITY;
-    int best_w = 0, best_p = 0;
-    for (int warps : kTuneWarps) {
-        for (int per_sm = 1; per_sm <= 4; per_sm++) {
-            b->tune_warps = warps;
-            b->tune_per_sm = per_sm;
-            s = batch_prepare(b, b->h_steps, kTuneSteps);
-            if (s) return s;
-            if (b->pulse_threads != warps * 32 || b->pulse_per_sm != per_sm) continue;
-            RSC_CUDA(batch_launch_pulse(b, 0));
-            RSC_CUDA(cudaEventRecord(ev.a, b->stream));
-            for (int r = 0; r < kTuneReps; r++) RSC_CUDA(batch_launch_pulse(b, 0));
-            RSC_CUDA(cudaEventRecord(ev.b, b->stream));
-            RSC_CUDA(cudaEventSynchronize(ev.b));
-            float ms = 0.0f;
-            RSC_CUDA(cudaEventElapsedTime(&ms, ev.a, ev.b));
-            b->launches += 1 + kTuneReps;
-            if (ms < best) {
-                best = ms;
-                best_w = warps;
-                best_p = per_sm;
-            }
-        }
+    {
+        BatchScratch c;
+        b->tuning = true;
+        s = batch_prepare(b, b->h_steps, batch_tune_steps(b));
+        if (s == RSC_OK) s = batch_tune_scratch(b, c);
+        if (s == RSC_OK) s = batch_tune_pulse(b, c, ev);
+        if (s == RSC_OK) s = batch_tune_advance(b, c, ev);
+        if (s == RSC_OK) s = batch_prepare(b, b->h_steps, batch_tune_steps(b));
+        b->tuning = false;
+        (void)cudaStreamSynchronize(b->stream);
     }
-    b->tune_warps = best_w;
-    b->tune_per_sm = best_p;
-    s = batch_prepare(b, b->h_steps, kTuneSteps);
-    if (s == RSC_OK) s = batch_tune_advance(b);
     if (s) return s;
     batch_drop_graph(b);
     RSC_CUDA(cudaEventRecord(b->ev_done, b->stream));
-    for (rsc_worker *x : b->w) RSC_CUDA(cudaStreamWaitEvent(x->stream, b->ev_done, 0));
+    for (rsc_worker *x : b->w) {
+        RSC_CUDA(cudaStreamWaitEvent(x->stream, b->ev_done, 0));
+        s = release_main(x);
+        if (s) return s;
+    }
     return RSC_OK;
 }
 
@@ -3350,6 +3387,13 @@ int rsc_batch_get_stream(rsc_batch *b, void **stream) {
 int rsc_batch_set_persistent(rsc_batch *b, int enable) {
     if (b == nullptr) return fail(RSC_ERR_ARG, "batch is NULL");
     b->persist = enable != 0;
+    return RSC_OK;
+}
+
+int rsc_batch_get_pulse_shape(rsc_batch *b, int *warps, int *blocks_per_sm) {
+    if (b == nullptr) return fail(RSC_ERR_ARG, "batch is NULL");
+    if (warps) *warps = b->pulse_threads / 32;
+    if (blocks_per_sm) *blocks_per_sm = b->pulse_per_sm;
     return RSC_OK;
 }
 

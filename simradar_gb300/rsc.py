@@ -129,6 +129,7 @@ def load_library():
         "rsc_batch_launch_count": ([P, ctypes.POINTER(ctypes.c_uint64)], I),
         "rsc_batch_get_stream": ([P, ctypes.POINTER(P)], I),
         "rsc_batch_get_shape": ([P, ctypes.POINTER(I), ctypes.POINTER(I)], I),
+        "rsc_batch_get_pulse_shape": ([P, ctypes.POINTER(I), ctypes.POINTER(I)], I),
     }
     for name, (argtypes, restype) in sig.items():
         fn = getattr(lib, name)
@@ -456,6 +457,13 @@ class Batch:
     def shape(self):
         wv, pv = ctypes.c_int(0), ctypes.c_int(0)
         _check(self._lib.rsc_batch_get_shape(self._h, ctypes.byref(wv), ctypes.byref(pv)))
+        return wv.value, pv.value
+
+    @property
+    def pulse_shape(self):
+        """Warps per block and blocks per SM of the latest run's pulses."""
+        wv, pv = ctypes.c_int(0), ctypes.c_int(0)
+        _check(self._lib.rsc_batch_get_pulse_shape(self._h, ctypes.byref(wv), ctypes.byref(pv)))
         return wv.value, pv.value
 
     def run(self, sim_descs, les_ids=None, out=None, use_graph=True, download=True, wait=True):
