@@ -737,10 +737,14 @@ double window_margin(double drift, float range_start, float range_delta, uint32_
 constexpr uint64_t kOrderedSteps = 256;
 constexpr int kNodeBatchSteps = 128;
 
-/* Gates from which compensated single scatterers meeting in L2 take less time
- * than every gate visited: the one shrinks with the nodes (2 M scatterers on
- * 77 gates 7.5 m apart 1875 us), the other grows with the gates (1670). */
-constexpr uint32_t kStrayGates = 82;
+/* Gates times half width from which compensated single scatterers meeting in L2
+ * take less time than every gate visited: the one goes with the scatterers per
+ * interval, which shrink as the gates do (2 M scatterers over 570 m, us: n = 4
+ * 1,873, n = 8 955, n = 12 645, n = 20 411, whatever the number of gates), the
+ * other with the gates (100 of them 2,148, 2,186, 2,186, 2,185).  They meet at
+ * 348; with 300,000 scatterers (n = 4 353 against 3.4 a gate, n = 8 157 against
+ * 3.5) at 390 and 360. */
+constexpr uint32_t kStrayWork = 360;
 
 /* A pulse through the node sums where the triangle allows them; the plain one
  * only where the triangle's ends meet the nodes (node_slip).
@@ -778,7 +782,7 @@ void use_nodes(rsc_worker *w, PulseArgs &P, int mode, bool batch) {
             P.any = batch ? 0 : 1;
             return;
         }
-        if (w->G < kStrayGates) return;
+        if (w->G * (uint32_t)n < kStrayWork) return;
     }
     P.mom_n = n;
     P.node = w->node + (rsc::kNodeMaxN - n);

@@ -156,3 +156,23 @@ def test_sums_at_the_ends_of_fp32(backend, r, x):
     if x < 1.0:
         assert ok.all()
     W.close()
+
+
+@pytest.mark.parametrize("spacing,gates", [(7.5, 89), (7.5, 90), (3.75, 44), (3.75, 45)])
+def test_out_of_order_on_fine_gates(backend, oracle_lib, spacing, gates):
+    """A state out of spatial order on gates too fine for moments, on both sides
+    of the line from which its scatterers go to their intervals one by one:
+    the bound of test_compensated_node_sums, 5e-9 of the sum of |w x| and the
+    output's rounding."""
+    O = oracle_lib
+    S = synth.make_scene(num_rain=20011, gates=gates, gate_spacing=spacing, les_count=1, seed=5)
+    W = backend.Worker(0)
+    synth.load_worker(W, S)
+    W.set_precision(1)
+    sd = synth.pulse_sim_desc(S, 50)
+    r64, ab = O.make_pulse_f64(O.OracleState(S.state), S, sd, return_abs=True)
+    for _ in range(2):
+        W.make_pulse(sd)
+        g = W.download_pulse(1.0).astype(np.float64)
+        assert (np.abs(g - r64) <= 5.0e-9 * ab + 6.0e-8 * np.abs(r64) + 1e-30).all()
+    W.close()
