@@ -607,7 +607,9 @@ __device__ __forceinline__ void node_gates(const PulseArgs &P, double *bins, uns
     /* the first of this thread's outputs' single contributions, on its way
      * together with the sums */
     double *extra = P.acc64 + (size_t)(MODE == 1 ? kCompSums : 4u) * nodes;
-    const double e0 = threadIdx.x < outs ? __ldcg(extra + threadIdx.x) : 0.0;
+    const unsigned first = MODE == 1 ? threadIdx.x : 2 * threadIdx.x;
+    const double e0 = first < outs ? __ldcg(extra + first) : 0.0;
+    const double f0 = MODE == 0 && first < outs ? __ldcg(extra + first + 1) : 0.0;
     if constexpr (MODE == 1) {
         const unsigned all = nodes * kCompSums;
 #pragma unroll 4
@@ -635,8 +637,7 @@ __device__ __forceinline__ void node_gates(const PulseArgs &P, double *bins, uns
     }
     /* each node's sum as a double-float, over bins[o], whose sums are out: the
      * FP64 units of the one block add 2 numbers a cycle (500,000 scatterers on
-     * 240 gates, 4 pulses: 178 us with FP64 sums here, 170 with these, 167 with
-     * FP32 ones) */
+     * 240 gates, 4 pulses: 138 us, 136 with FP32 sums) */
     float2 *sums = reinterpret_cast<float2 *>(bins);
     float *at_node = reinterpret_cast<float *>(sums + 4 * nodes);
     const unsigned copies = node_copies(P.G, P.mom_n);
@@ -672,27 +673,32 @@ __device__ __forceinline__ void node_gates(const PulseArgs &P, double *bins, uns
         __syncthreads();
     }
     for (unsigned o = threadIdx.x; o < nodes * 4; o += blockDim.x) P.acc64[o] = 0.0;
-    for (unsigned o = threadIdx.x; STRAY && o < 4 * nodes * copies; o += blockDim.x) P.stray[o] = 0.0;
+    for (unsigned o = threadIdx.x; STRAY && o < 2 * nodes * copies; o += blockDim.x) {
+        reinterpret_cast<double2 *>(P.stray)[o] = make_double2(0.0, 0.0);
+    }
+    /* two values of a gate per thread, which share its weights */
     const int n = P.mom_n;
-    for (unsigned o = threadIdx.x; o < outs; o += blockDim.x) {
-        const unsigned k = o >> 2, l = o & 3u;
+    const float4 *two = reinterpret_cast<const float4 *>(sums);
+    for (unsigned o = threadIdx.x; o < P.G * 2; o += blockDim.x) {
+        const unsigned k = o >> 1, half = o & 1u;
         const float rk = __ldg(P.rk + k);
-        float sum = 0.0f, low = 0.0f;
+        float sum[2] = {0.0f, 0.0f}, low[2] = {0.0f, 0.0f};
         const unsigned end = min(k + 2u * (unsigned)n + 1u, nodes);
 #pragma unroll 4
         for (unsigned at = k; at < end; at++) {
             const float w = fmaxf(1.0f - fabsf(at_node[at] - rk) * P.rwd[0], 0.0f);
-            float a, b;
-            df_mul_pair(sums[4 * at + l].x, sums[4 * at + l].y, w, 0.0f, a, b);
-            df_acc(sum, low, a, b);
+            const float4 x = two[2 * at + half];
+            const float a = x.x * w, b = x.z * w;
+            df_acc(sum[0], low[0], a, fmaf(x.y, w, fmaf(x.x, w, -a)));
+            df_acc(sum[1], low[1], b, fmaf(x.w, w, fmaf(x.z, w, -b)));
         }
-        sum = sum + low;
-        const double e = o == threadIdx.x ? e0 : __ldcg(extra + o);
-        if (not_zero(e)) {
-            sum = (float)((double)sum + e);   /* not finite */
-            extra[o] = 0.0;
+        float2 g = make_float2(sum[0] + low[0], sum[1] + low[1]);
+        const double e = o == threadIdx.x ? e0 : __ldcg(extra + 2 * o), f = o == threadIdx.x ? f0 : __ldcg(extra + 2 * o + 1);
+        if (not_zero(e) || not_zero(f)) {   /* not finite */
+            g = make_float2((float)((double)g.x + e), (float)((double)g.y + f));
+            extra[2 * o] = extra[2 * o + 1] = 0.0;
         }
-        reinterpret_cast<float *>(P.pulse)[o] = sum;
+        reinterpret_cast<float2 *>(P.pulse)[o] = g;
     }
     if (threadIdx.x == 0) *P.counter = 0u;
 }
