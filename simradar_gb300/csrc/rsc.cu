@@ -689,6 +689,11 @@ int node_span(const PulseArgs &P) {
  * 9.6e-3 at 60 km), and every scatterer of an end's interval would have that
  * weight too much or too little. */
 double node_slip(float start, float delta, uint32_t G, int n, float scale) {
+    /* a start and a spacing that are multiples of the last node's ulp: every
+     * origin and node is exact */
+    const double far = std::max(fabs((double)start - n * (double)delta), fabs((double)start + ((double)G - 1 + n) * (double)delta));
+    const double ulp = ldexp(1.0, ilogb(far) - 23), a = (double)start / ulp, b = (double)delta / ulp;
+    if (far > 0.0 && a == floor(a) && b == floor(b)) return fabs(n * (double)delta * (double)scale - 1.0);
     std::vector<float> rk(G);
     float r = start;
     for (uint32_t k = 0; k < G; k++) {
