@@ -451,7 +451,7 @@ def bench_batch(torch, rsc, synth, dev, steps):
     res["speedup_vs_back_to_back_no_download"] = bg / res["back_to_back"]["pulses_per_s_no_download"]
     res["workload"] = ("64 instances, scatterers log-uniform 65,536-4,194,304 (total %d), debris 0-4096 per type, "
                        "Marshall-Palmer N0 4000-16000, PPI / RHI alternating, %d gates, compensated form; %d steps "
-                       "timed per instance.  Every pulse reaches the host in both: batched, one copy per run; back "
+                       "timed per instance.  Every pulse reaches the host in both: batched, one copy per part of a run; back "
                        "to back, each pulse copied to page-locked memory in stream order with one wait per "
                        "instance (speedup_vs_back_to_back).  Secondary: back to back with a blocking read of every "
                        "pulse as rs.c does, and with no pulse copied" % (total, GATES, steps))

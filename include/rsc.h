@@ -39,7 +39,11 @@ extern "C" {
 #define RSC_MAX_GATES 512       /* RS_MAX_GATES, rs_const.h:22 */
 
 /* pulse-formation precision (additive; the reference has only RSC_PULSE_PLAIN) */
-#define RSC_PULSE_PLAIN 0       /* FP32 exactly as rs.cl scat_sig_aux + pass 1 (gate weights bit-exact) */
+/* FP32 as rs.cl scat_sig_aux + pass 1.  On a triangle of a whole number of gate
+ * spacings whose ends meet the gate origins to 2^-23 of a weight, the gate
+ * weights are interpolated between those origins (within 2.5e-7); everywhere
+ * else, and in pulses that write aux / sig, they are pass 1's bit for bit. */
+#define RSC_PULSE_PLAIN 0
 #define RSC_PULSE_COMPENSATED 1 /* double-float terms (split range phase), FP64 gate origins, error-free sums */
 #define RSC_PULSE_F64 2         /* FP64 reference of the same FP32 state (error metric oracle) */
 
